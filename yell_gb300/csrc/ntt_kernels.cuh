@@ -22,6 +22,7 @@
 #pragma once
 #include <atomic>
 #include <cstring>
+#include <type_traits>
 #include <utility>
 
 #include "kernels.h"
@@ -446,12 +447,12 @@ __global__ void __launch_bounds__(C::THREADS) k_row_pass(LimbSet ls, const DevMo
   extern __shared__ __align__(16) uint64_t smem[];
   constexpr int K = C::K, NR = C::NR;
   constexpr uint32_t log_n = K + K1;
-  constexpr int TPL = log_n - kTileLog;
+  constexpr int TPL = log_n - C::T;
   grid_dep_launch();
   grid_dep_wait();  // as in k_col_pass
   const uint32_t tid = threadIdx.x;
   const uint32_t limb = ls.ordered(blockIdx.x >> TPL);
-  const uint32_t off = (blockIdx.x & ((1u << TPL) - 1u)) << kTileLog;
+  const uint32_t off = (blockIdx.x & ((1u << TPL) - 1u)) << C::T;
   uint64_t* data = ls.limb(limb, log_n) + off;
   const DevMod m = load_mod(mods, ls.cm(limb));
   const uint32_t G = (off >> K) + C::sub(tid);
@@ -604,7 +605,7 @@ __device__ __forceinline__ void col_pass2_body(ConstLimbSet a, ConstLimbSet b, L
   constexpr uint32_t log_n = K + LOGB;
   constexpr int TPL = LOGB - LB;
   uint64_t* sa = smem;
-  uint64_t* sb = smem + tile_smem_words(1u << kTileLog);
+  uint64_t* sb = smem + tile_smem_words(1u << C::T);
   const uint32_t tid = threadIdx.x;
   const uint32_t limb = ca.ordered(bid >> TPL);
   const uint32_t col0 = (bid & ((1u << TPL) - 1u)) << LB;
@@ -635,8 +636,15 @@ __device__ __forceinline__ void col_pass2_body(ConstLimbSet a, ConstLimbSet b, L
   }
 }
 
+// Resident threads per SM that the two-operand kernels are compiled for: 512
+// (128 registers) at 16 words of each operand per thread, 768 (80 registers)
+// at 8 or 4 (512 limbs of 2^16 at k1 = 8, tiles of 2^10: 1067 us compiled for
+// 512, 1022 for 768, 1036 for 1024).
+template <class C>
+constexpr int two_operand_threads() { return C::LOGE == 4 ? 512 : 768; }
+
 template <class C, int LOGB>
-__global__ void __launch_bounds__(C::THREADS, min_blocks(512, C::THREADS))
+__global__ void __launch_bounds__(C::THREADS, min_blocks(two_operand_threads<C>(), C::THREADS))
     k_col_pass2(ConstLimbSet a, ConstLimbSet b, LimbSet ca, LimbSet cb, const DevMod* __restrict__ mods) {
   grid_dep_launch();
   grid_dep_wait();  // as in k_col_pass
@@ -653,12 +661,12 @@ __device__ __forceinline__ void polymul_rows_body(LimbSet ca, ConstLimbSet sbuf,
   // rows stay with their threads: barriers over a row's threads only
   constexpr int BK = C::LOCAL_BARRIER;
   constexpr uint32_t log_n = K + K1;
-  constexpr int TPL = log_n - kTileLog;
+  constexpr int TPL = log_n - C::T;
   uint64_t* sa = smem;
-  uint64_t* sb = smem + tile_smem_words(1u << kTileLog);
+  uint64_t* sb = smem + tile_smem_words(1u << C::T);
   const uint32_t tid = threadIdx.x;
   const uint32_t limb = ca.ordered(bid >> TPL);
-  const uint32_t off = (bid & ((1u << TPL) - 1u)) << kTileLog;
+  const uint32_t off = (bid & ((1u << TPL) - 1u)) << C::T;
   uint64_t* pa = ca.limb(limb, log_n) + off;
   const uint64_t* pb = sbuf.limb(limb, log_n) + off;
   const DevMod m = load_mod(mods, ca.cm(limb));
@@ -689,7 +697,7 @@ __device__ __forceinline__ void polymul_rows_body(LimbSet ca, ConstLimbSet sbuf,
 }
 
 template <class C, int K1>
-__global__ void __launch_bounds__(C::THREADS, min_blocks(512, C::THREADS))
+__global__ void __launch_bounds__(C::THREADS, min_blocks(two_operand_threads<C>(), C::THREADS))
     k_polymul_rows(LimbSet ca, ConstLimbSet sbuf, const DevMod* __restrict__ mods) {
   grid_dep_launch();
   grid_dep_wait();  // as in k_col_pass
@@ -739,7 +747,7 @@ __global__ void __launch_bounds__(C::THREADS, min_blocks(512, C::THREADS))
   constexpr int TPL = LOGB - LB;
   static_assert(NR >= 2, "the last round reads shared memory before the next tile is staged");
   uint64_t* sa = smem;
-  uint64_t* sb = smem + tile_smem_words(1u << kTileLog);
+  uint64_t* sb = smem + tile_smem_words(1u << C::T);
   const uint32_t tid = threadIdx.x;
   constexpr int E = 1 << C::LOGE;
   uint64_t xa[E], xb[E];
@@ -790,9 +798,9 @@ __global__ void __launch_bounds__(C::THREADS, min_blocks(512, C::THREADS))
   constexpr int K = C::K, NR = C::NR;
   constexpr int BK = C::LOCAL_BARRIER;
   constexpr uint32_t log_n = K + K1;
-  constexpr int TPL = log_n - kTileLog;
+  constexpr int TPL = log_n - C::T;
   uint64_t* sa = smem;
-  uint64_t* sb = smem + tile_smem_words(1u << kTileLog);
+  uint64_t* sb = smem + tile_smem_words(1u << C::T);
   const uint32_t tid = threadIdx.x;
   constexpr int E = 1 << C::LOGE;
   uint64_t xa[E], xb[E];
@@ -905,22 +913,24 @@ cudaError_t set_smem(KernelT kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-// Whole-limb tile: 2^T words (T >= log_n); 16 words per thread (8 at N = 8).
-template <int LOGN, int T>
-using WholeCfg = TileCfg<T, LOGN, 0, (LOGN >= 4 ? 4 : 3)>;
+// Whole-limb tile: 2^T words (T >= log_n); 16 words per thread (8 at N = 8)
+// unless a variant for few limbs takes fewer.
+constexpr int whole_loge(int log_n) { return log_n >= 4 ? 4 : 3; }
+template <int LOGN, int T, int LOGE = whole_loge(LOGN)>
+using WholeCfg = TileCfg<T, LOGN, 0, LOGE>;
 // Two-pass tiles: 4096 words, 2^LOGE words per thread per round (radix-2^LOGE
 // rounds): LOGE = 4 is 256 threads, LOGE = 3 is 512 threads per tile.
-template <int LOGN, int K1, int LOGE = 4>
-using ColCfg = TileCfg<kTileLog, K1, kTileLog - K1, LOGE>;
-template <int LOGN, int K1, int LOGE = 4>
-using RowCfg = TileCfg<kTileLog, LOGN - K1, 0, LOGE>;
+template <int LOGN, int K1, int LOGE = 4, int T = kTileLog>
+using ColCfg = TileCfg<T, K1, T - K1, LOGE>;
+template <int LOGN, int K1, int LOGE = 4, int T = kTileLog>
+using RowCfg = TileCfg<T, LOGN - K1, 0, LOGE>;
 
 constexpr size_t tile_bytes(int T) { return tile_smem_words(1u << T) * sizeof(uint64_t); }
 constexpr size_t kTileSmemBytes = tile_bytes(kTileLog);
 
-template <int LOGN, int T>
+template <int LOGN, int T, int LOGE>
 cudaError_t launch_whole_ntt(const LimbSet& ls, const DevMod* mods, NttDir dir, cudaStream_t st) {
-  using C = WholeCfg<LOGN, T>;
+  using C = WholeCfg<LOGN, T, LOGE>;
   const uint32_t per = 1u << (T - LOGN);
   const uint32_t grid = (ls.count + per - 1) / per;
   const size_t smem = tile_bytes(T);
@@ -934,11 +944,11 @@ cudaError_t launch_whole_ntt(const LimbSet& ls, const DevMod* mods, NttDir dir, 
   return cudaGetLastError();
 }
 
-template <int LOGN, int T>
+template <int LOGN, int T, int LOGE>
 cudaError_t launch_whole_polymul(const LimbSet& c, const ConstLimbSet& a, const ConstLimbSet& b,
                                  const DevMod* mods, uint64_t*, uint64_t* const*, cudaStream_t st) {
   mods += kPolymulConsts;  // the fused polymul's copy of the constants
-  using C = WholeCfg<LOGN, T>;
+  using C = WholeCfg<LOGN, T, LOGE>;
   const uint32_t per = 1u << (T - LOGN);
   const uint32_t grid = (c.count + per - 1) / per;
   LaunchScope ps("polymul_whole", st);
@@ -947,9 +957,9 @@ cudaError_t launch_whole_polymul(const LimbSet& c, const ConstLimbSet& a, const 
   return cudaGetLastError();
 }
 
-template <int LOGN, int T>
+template <int LOGN, int T, int LOGE>
 cudaError_t set_attrs_whole() {
-  using C = WholeCfg<LOGN, T>;
+  using C = WholeCfg<LOGN, T, LOGE>;
   const size_t s = tile_bytes(T);
   cudaError_t e;
   if ((e = set_smem(k_ntt_whole<C, 0>, s)) != cudaSuccess) return e;
@@ -958,73 +968,123 @@ cudaError_t set_attrs_whole() {
   return set_smem(k_polymul_whole<C>, 2 * s);
 }
 
-template <int LOGN, int K1, int LC = 4, int LR = 4>
+// Tiles of the two-pass kernels of a split.  TwoPassTiles<LOGN, K1> is the one
+// for calls that fill the chip: each kernel has the tile and the words per
+// thread that ran fastest for it, measured apart from the others.  Fewer
+// words per tile mean more, smaller CTAs (a shorter last wave, and a CTA's
+// loads overlap more other CTAs' arithmetic) and more sectors per word in the
+// column passes; fewer words per thread more exchanges.  GB300, 512 limbs of
+// 2^16 at k1 = 7, tiles of 2^12 with 16 words per thread -> the tile below:
+// forward column pass 156 -> 147 us, forward row pass 225 -> 206, inverse row
+// pass 276 -> 233, inverse column pass 173 -> 163 (polymul 170 -> 160); 512
+// limbs of 2^14: polymul's forward column pass 87 -> 80.  Only the fused row
+// step (16 words of two operands per thread) wants its 2^12 tile: 566 us
+// against 580 at 8 words per thread and 680 at 2^10 and 2^11 words.
+constexpr int tile_log(int want, int least) { return want > least ? want : least; }
+
+template <int LOGN, int K1>
+struct TwoPassTiles {
+  static constexpr int K = LOGN - K1;
+  // the column tiles keep at least 2^2 columns (32-byte sectors)
+  using Col2 = ColCfg<LOGN, K1, (LOGN <= 15 ? 3 : 4), (LOGN <= 15 ? tile_log(10, K1 + 2) : kTileLog)>;
+  using Rows = RowCfg<LOGN, K1>;
+  using ColFwd = ColCfg<LOGN, K1, 4, tile_log(11, K1 + 2)>;
+  using ColInv = ColFwd;
+  using RowFwd = RowCfg<LOGN, K1, 4, tile_log(10, K)>;
+  using RowInv = RowCfg<LOGN, K1, (K <= 8 ? 3 : 4), tile_log(10, K)>;
+};
+
+// The same tile log and words per thread for every kernel: 2^12-word tiles
+// with other round widths, and the small tiles of calls with few limbs.
+template <int LOGN, int K1, int LC, int LR, int T>
+struct UniformTiles {
+  using Col2 = ColCfg<LOGN, K1, LC, T>;
+  using ColFwd = Col2;
+  using ColInv = Col2;
+  using Rows = RowCfg<LOGN, K1, LR, T>;
+  using RowFwd = Rows;
+  using RowInv = Rows;
+};
+
+template <class C>
+constexpr size_t cfg_bytes() { return tile_bytes(C::T); }
+
+template <int LOGN, int K1, class TT>
 cudaError_t launch_two_pass_ntt(const LimbSet& ls, const DevMod* mods, NttDir dir, cudaStream_t st) {
   constexpr int LOGB = LOGN - K1;
-  using CC = ColCfg<LOGN, K1, LC>;
-  using RC = RowCfg<LOGN, K1, LR>;
-  const uint32_t tiles = ls.count << (LOGN - kTileLog);
   const ConstLimbSet cls = as_const(ls);
   if (dir == NttDir::kBackward) {
+    using RC = typename TT::RowInv;
+    using CC = typename TT::ColInv;
     {
       LaunchScope ps("row_pass_inv", st);
-      launch_dependent(k_row_pass<RC, K1, true>, tiles, RC::THREADS, kTileSmemBytes, st, ls, mods, 0);
+      launch_dependent(k_row_pass<RC, K1, true>, ls.count << (LOGN - RC::T), RC::THREADS, cfg_bytes<RC>(), st, ls, mods,
+                       0);
     }
     LaunchScope ps("col_pass_inv", st);
-    launch_dependent(k_col_pass<CC, LOGB, true>, tiles, CC::THREADS, kTileSmemBytes, st, cls, ls, mods);
+    launch_dependent(k_col_pass<CC, LOGB, true>, ls.count << (LOGN - CC::T), CC::THREADS, cfg_bytes<CC>(), st, cls, ls,
+                     mods);
   } else {
+    using RC = typename TT::RowFwd;
+    using CC = typename TT::ColFwd;
     {
       LaunchScope ps("col_pass_fwd", st);
-      launch_dependent(k_col_pass<CC, LOGB, false>, tiles, CC::THREADS, kTileSmemBytes, st, cls, ls, mods);
+      launch_dependent(k_col_pass<CC, LOGB, false>, ls.count << (LOGN - CC::T), CC::THREADS, cfg_bytes<CC>(), st, cls,
+                       ls, mods);
     }
     LaunchScope ps("row_pass_fwd", st);
-    launch_dependent(k_row_pass<RC, K1, false>, tiles, RC::THREADS, kTileSmemBytes, st, ls, mods,
+    launch_dependent(k_row_pass<RC, K1, false>, ls.count << (LOGN - RC::T), RC::THREADS, cfg_bytes<RC>(), st, ls, mods,
                      dir == NttDir::kForward ? 1 : 0);
   }
   g_kernel_launches += 2;
   return cudaGetLastError();
 }
 
-template <int LOGN, int K1, int LC = 4, int LR = 4>
+template <int LOGN, int K1, class TT>
 cudaError_t launch_two_pass_polymul(const LimbSet& c, const ConstLimbSet& a, const ConstLimbSet& b,
                                     const DevMod* mods, uint64_t* scratch, uint64_t* const* scratch_ptrs,
                                     cudaStream_t st) {
   mods += kPolymulConsts;  // the fused polymul's copy of the constants
   constexpr int LOGB = LOGN - K1;
-  using CC = ColCfg<LOGN, K1, LC>;
-  using RC = RowCfg<LOGN, K1, LR>;
-  const uint32_t tiles = c.count << (LOGN - kTileLog);
+  using C2 = typename TT::Col2;
+  using RC = typename TT::Rows;
+  using CC = typename TT::ColInv;
   LimbSet sl = c;
   sl.base = scratch_ptrs ? nullptr : scratch;
   sl.ptrs = scratch_ptrs;
   {
     LaunchScope ps("polymul_col_fwd", st);
-    launch_dependent(k_col_pass2<CC, LOGB>, tiles, CC::THREADS, 2 * kTileSmemBytes, st, a, b, c, sl, mods);
+    launch_dependent(k_col_pass2<C2, LOGB>, c.count << (LOGN - C2::T), C2::THREADS, 2 * cfg_bytes<C2>(), st, a, b, c,
+                     sl, mods);
   }
   {
     LaunchScope ps("polymul_rows", st);
-    launch_dependent(k_polymul_rows<RC, K1>, tiles, RC::THREADS, 2 * kTileSmemBytes, st, c, as_const(sl), mods);
+    launch_dependent(k_polymul_rows<RC, K1>, c.count << (LOGN - RC::T), RC::THREADS, 2 * cfg_bytes<RC>(), st, c,
+                     as_const(sl), mods);
   }
   {
     LaunchScope ps("polymul_col_inv", st);
-    launch_dependent(k_col_pass<CC, LOGB, true>, tiles, CC::THREADS, kTileSmemBytes, st, as_const(c), c, mods);
+    launch_dependent(k_col_pass<CC, LOGB, true>, c.count << (LOGN - CC::T), CC::THREADS, cfg_bytes<CC>(), st,
+                     as_const(c), c, mods);
   }
   g_kernel_launches += 3;
   return cudaGetLastError();
 }
 
-template <int LOGN, int K1, int LC = 4, int LR = 4>
+template <int LOGN, int K1, class TT>
 cudaError_t set_attrs_two_pass() {
   constexpr int LOGB = LOGN - K1;
-  using CC = ColCfg<LOGN, K1, LC>;
-  using RC = RowCfg<LOGN, K1, LR>;
   cudaError_t e;
-  if ((e = set_smem(k_col_pass<CC, LOGB, false>, kTileSmemBytes)) != cudaSuccess) return e;
-  if ((e = set_smem(k_col_pass<CC, LOGB, true>, kTileSmemBytes)) != cudaSuccess) return e;
-  if ((e = set_smem(k_row_pass<RC, K1, false>, kTileSmemBytes)) != cudaSuccess) return e;
-  if ((e = set_smem(k_row_pass<RC, K1, true>, kTileSmemBytes)) != cudaSuccess) return e;
-  if ((e = set_smem(k_col_pass2<CC, LOGB>, 2 * kTileSmemBytes)) != cudaSuccess) return e;
-  return set_smem(k_polymul_rows<RC, K1>, 2 * kTileSmemBytes);
+  if ((e = set_smem(k_col_pass<typename TT::ColFwd, LOGB, false>, cfg_bytes<typename TT::ColFwd>())) != cudaSuccess)
+    return e;
+  if ((e = set_smem(k_col_pass<typename TT::ColInv, LOGB, true>, cfg_bytes<typename TT::ColInv>())) != cudaSuccess)
+    return e;
+  if ((e = set_smem(k_row_pass<typename TT::RowFwd, K1, false>, cfg_bytes<typename TT::RowFwd>())) != cudaSuccess)
+    return e;
+  if ((e = set_smem(k_row_pass<typename TT::RowInv, K1, true>, cfg_bytes<typename TT::RowInv>())) != cudaSuccess)
+    return e;
+  if ((e = set_smem(k_col_pass2<typename TT::Col2, LOGB>, 2 * cfg_bytes<typename TT::Col2>())) != cudaSuccess) return e;
+  return set_smem(k_polymul_rows<typename TT::Rows, K1>, 2 * cfg_bytes<typename TT::Rows>());
 }
 
 // Persistent grid of a pipelined kernel: its resident CTAs on this device,
@@ -1080,20 +1140,20 @@ cudaError_t set_attrs_two_pass_pipe() {
   using CC = ColCfg<LOGN, K1, LC>;
   using RC = RowCfg<LOGN, K1, LR>;
   cudaError_t e;
-  if ((e = set_attrs_two_pass<LOGN, K1, LC, LR>()) != cudaSuccess) return e;
+  if ((e = set_attrs_two_pass<LOGN, K1, TwoPassTiles<LOGN, K1>>()) != cudaSuccess) return e;
   if ((e = set_smem(k_col_pass2_pipe<CC, LOGB>, 2 * kTileSmemBytes)) != cudaSuccess) return e;
   if ((e = set_smem(k_polymul_rows_pipe<RC, K1>, 2 * kTileSmemBytes)) != cudaSuccess) return e;
   return set_smem(k_col_inv_pipe<CC, LOGB>, kTileSmemBytes);
 }
 
-template <int LOGN, int T>
+template <int LOGN, int T, int LOGE = whole_loge(LOGN)>
 Variant whole_variant() {
   Variant v;
-  std::snprintf(v.name, sizeof(v.name), "whole-limb tile 2^%d (%d threads, %d limbs/CTA)", T,
-                1 << (T - (LOGN >= 4 ? 4 : 3)), 1 << (T - LOGN));
-  v.ntt = &launch_whole_ntt<LOGN, T>;
-  v.polymul = &launch_whole_polymul<LOGN, T>;
-  v.set_attrs = &set_attrs_whole<LOGN, T>;
+  std::snprintf(v.name, sizeof(v.name), "whole-limb tile 2^%d (%d threads, %d limbs/CTA)", T, 1 << (T - LOGE),
+                1 << (T - LOGN));
+  v.ntt = &launch_whole_ntt<LOGN, T, LOGE>;
+  v.polymul = &launch_whole_polymul<LOGN, T, LOGE>;
+  v.set_attrs = &set_attrs_whole<LOGN, T, LOGE>;
   v.ntt_launches = 1;
   v.polymul_launches = 1;
   return v;
@@ -1101,20 +1161,36 @@ Variant whole_variant() {
 
 // Named "two-pass k1=K1 (...)"; variants whose column or row tiles use other
 // than 16 words per thread name both word counts.
+template <int LOGN, int K1, class TT>
+Variant two_pass_of() {
+  Variant v;
+  v.ntt = &launch_two_pass_ntt<LOGN, K1, TT>;
+  v.polymul = &launch_two_pass_polymul<LOGN, K1, TT>;
+  v.set_attrs = &set_attrs_two_pass<LOGN, K1, TT>;
+  v.ntt_launches = 2;
+  v.polymul_launches = 3;
+  v.polymul_scratch = true;
+  return v;
+}
+
 template <int LOGN, int K1, int LC = 4, int LR = 4>
 Variant two_pass_variant() {
-  Variant v;
+  using TT = std::conditional_t<LC == 4 && LR == 4, TwoPassTiles<LOGN, K1>, UniformTiles<LOGN, K1, LC, LR, kTileLog>>;
+  Variant v = two_pass_of<LOGN, K1, TT>();
   if (LC == 4 && LR == 4)
     std::snprintf(v.name, sizeof(v.name), "two-pass k1=%d (columns of 2^%d, rows of 2^%d)", K1, K1, LOGN - K1);
   else
     std::snprintf(v.name, sizeof(v.name), "two-pass k1=%d (columns of 2^%d, rows of 2^%d; %d/%d words per thread)",
                   K1, K1, LOGN - K1, 1 << LC, 1 << LR);
-  v.ntt = &launch_two_pass_ntt<LOGN, K1, LC, LR>;
-  v.polymul = &launch_two_pass_polymul<LOGN, K1, LC, LR>;
-  v.set_attrs = &set_attrs_two_pass<LOGN, K1, LC, LR>;
-  v.ntt_launches = 2;
-  v.polymul_launches = 3;
-  v.polymul_scratch = true;
+  return v;
+}
+
+// Small tiles with few words per thread, for calls with few limbs.
+template <int LOGN, int K1, int LOGE, int T>
+Variant two_pass_few_variant() {
+  Variant v = two_pass_of<LOGN, K1, UniformTiles<LOGN, K1, LOGE, LOGE, T>>();
+  std::snprintf(v.name, sizeof(v.name), "two-pass k1=%d (columns of 2^%d, rows of 2^%d; %d words per thread, tiles of 2^%d)",
+                K1, K1, LOGN - K1, 1 << LOGE, T);
   return v;
 }
 
