@@ -88,6 +88,7 @@ int num_sms() {
 
 std::vector<Variant> g_table[kMaxLogN + 1];
 std::once_flag g_table_once;
+// Selected variant + 1, or 0 when none was selected.
 std::array<std::array<std::atomic<uint8_t>, kMaxLogN + 1>, 64> g_selected{};
 
 void build_table() {
@@ -98,6 +99,10 @@ void build_table() {
   add_two_pass_variants_c(g_table);
   add_two_pass_variants_d(g_table);
   add_two_pass_variants_e(g_table);
+  // after the others: a variant keeps its index
+  add_few_limb_variants(g_table);
+  add_two_pass_few_variants(g_table);
+  add_cluster_variants(g_table);
 }
 
 int current_device() {
@@ -106,10 +111,16 @@ int current_device() {
   return (d >= 0 && d < 64) ? d : 0;
 }
 
-const Variant& pick(uint32_t log_n) {
+// The variant a call of `limbs` limbs runs: the selected one, else the one
+// registered for that many limbs, else the first.
+const Variant& pick(uint32_t log_n, uint32_t limbs, uint32_t Variant::*bound) {
   const std::vector<Variant>& vs = variants_of(log_n);
-  const uint32_t v = selected_variant(current_device(), log_n);
-  return vs[v < vs.size() ? v : 0];
+  const uint32_t sel = g_selected[current_device()][log_n].load(std::memory_order_relaxed);
+  if (sel != 0 && sel <= vs.size()) return vs[sel - 1];
+  const Variant* best = &vs[0];
+  for (const Variant& v : vs)
+    if (v.*bound >= limbs && (best->*bound < limbs || v.*bound < best->*bound)) best = &v;
+  return *best;
 }
 
 }  // namespace
@@ -120,11 +131,12 @@ const std::vector<Variant>& variants_of(uint32_t log_n) {
 }
 
 uint32_t selected_variant(int device, uint32_t log_n) {
-  return g_selected[device][log_n].load(std::memory_order_relaxed);
+  const uint32_t sel = g_selected[device][log_n].load(std::memory_order_relaxed);
+  return sel != 0 ? sel - 1 : 0;
 }
 
 void select_variant(int device, uint32_t log_n, uint32_t v) {
-  g_selected[device][log_n].store((uint8_t)v, std::memory_order_relaxed);
+  g_selected[device][log_n].store((uint8_t)(v + 1), std::memory_order_relaxed);
 }
 
 cudaError_t init_kernel_attributes() {
@@ -136,8 +148,12 @@ cudaError_t init_kernel_attributes() {
   return cudaSuccess;
 }
 
-uint32_t ntt_launch_count(uint32_t log_n, const NttShape&) { return pick(log_n).ntt_launches; }
-uint32_t polymul_launch_count(uint32_t log_n, const NttShape&) { return pick(log_n).polymul_launches; }
+uint32_t ntt_launch_count(uint32_t log_n, const NttShape&) {
+  return variants_of(log_n)[selected_variant(current_device(), log_n)].ntt_launches;
+}
+uint32_t polymul_launch_count(uint32_t log_n, const NttShape&) {
+  return variants_of(log_n)[selected_variant(current_device(), log_n)].polymul_launches;
+}
 
 // The words a polymul of this degree may need, whichever variant is selected
 // (the selection can change between the caller's allocation and its call).
@@ -152,7 +168,7 @@ size_t polymul_scratch_words(uint32_t count, uint32_t log_n, const NttShape&) {
 bool polymul_scratch_optional(uint32_t log_n) {
   if (log_n < kMinLogN || log_n > kMaxLogN) return true;
   for (const Variant& v : variants_of(log_n))
-    if (!v.polymul_scratch) return true;
+    if (!v.polymul_scratch && !v.few_limbs) return true;
   return false;
 }
 
@@ -160,7 +176,7 @@ cudaError_t launch_ntt(const LimbSet& ls, uint32_t log_n, const DevMod* mods, Nt
                        const NttShape&, cudaStream_t st) {
   if (ls.count == 0) return cudaSuccess;
   if (log_n < kMinLogN || log_n > kMaxLogN) return cudaErrorInvalidValue;
-  return pick(log_n).ntt(ls, mods, dir, st);
+  return pick(log_n, ls.count, &Variant::ntt_upto).ntt(ls, mods, dir, st);
 }
 
 cudaError_t launch_polymul(const LimbSet& c, const ConstLimbSet& a, const ConstLimbSet& b,
@@ -168,12 +184,12 @@ cudaError_t launch_polymul(const LimbSet& c, const ConstLimbSet& a, const ConstL
                            const NttShape&, cudaStream_t st, uint64_t* const* scratch_ptrs) {
   if (c.count == 0) return cudaSuccess;
   if (log_n < kMinLogN || log_n > kMaxLogN) return cudaErrorInvalidValue;
-  const Variant* v = &pick(log_n);
+  const Variant* v = &pick(log_n, c.count, &Variant::polymul_upto);
   if (v->polymul_scratch && scratch == nullptr && scratch_ptrs == nullptr) {
     // Without scratch, the first (selection order) variant that needs none.
     v = nullptr;
     for (const Variant& w : variants_of(log_n))
-      if (!w.polymul_scratch) {
+      if (!w.polymul_scratch && !w.few_limbs) {
         v = &w;
         break;
       }

@@ -4,8 +4,11 @@
 // butterflies (so produce the same words) with a different split of the work:
 // the tile size of the whole-limb path (limbs per CTA) or the number of
 // column stages k1 of the two-pass path (columns of 2^k1 words, rows of
-// 2^(log_n - k1) words).  Variant 0 is the default; the autotuner times every
-// variant of a degree on the current device and keeps the fastest.
+// 2^(log_n - k1) words), or one limb per thread-block cluster.  A degree for
+// which no variant was selected takes the one registered for the call's
+// number of limbs (polymul_upto, ntt_upto), else variant 0; the autotuner
+// times every variant of a degree on the current device and selects the
+// fastest, which then runs at every number of limbs.
 #pragma once
 #include <vector>
 
@@ -22,7 +25,23 @@ struct Variant {
   uint32_t ntt_launches = 0;
   uint32_t polymul_launches = 0;
   bool polymul_scratch = false;  // the polymul needs one operand's worth of scratch words
+  // Chosen without a selection for calls of at most this many limbs (0:
+  // never); among several, the one with the smallest such bound.
+  uint32_t polymul_upto = 0, ntt_upto = 0;
+  // One of the variants for few limbs: never the stand-in for a polymul
+  // called without scratch.
+  bool few_limbs = false;
 };
+
+constexpr uint32_t kAnyLimbs = 0xFFFFFFFFu;
+
+// A variant for few limbs, with its bounds.
+inline Variant upto(Variant v, uint32_t polymul_limbs, uint32_t ntt_limbs) {
+  v.polymul_upto = polymul_limbs;
+  v.ntt_upto = ntt_limbs;
+  v.few_limbs = true;
+  return v;
+}
 
 // Registration, one per translation unit (by_degree has kMaxLogN + 1 entries).
 void add_whole_variants_small(std::vector<Variant>* by_degree);  // 2^3 .. 2^8
@@ -33,8 +52,13 @@ void add_two_pass_variants_c(std::vector<Variant>* by_degree);   // 2^18 .. 2^20
 void add_two_pass_variants_d(std::vector<Variant>* by_degree);   // more 2^16 splits and round widths
 void add_two_pass_variants_e(std::vector<Variant>* by_degree);   // pipelined polymul, 2^16
 
+void add_few_limb_variants(std::vector<Variant>* by_degree);     // 2^6 .. 2^10, whole-limb, fewer words per thread
+void add_two_pass_few_variants(std::vector<Variant>* by_degree); // 2^13 .. 2^20, small tiles
+void add_cluster_variants(std::vector<Variant>* by_degree);      // 2^10 .. 2^14, one limb per cluster
+
 // Variant table of a degree, and the variant selected on the current device.
 const std::vector<Variant>& variants_of(uint32_t log_n);
+// (0 when none was).
 uint32_t selected_variant(int device, uint32_t log_n);
 void select_variant(int device, uint32_t log_n, uint32_t v);
 

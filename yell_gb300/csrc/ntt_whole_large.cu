@@ -1,6 +1,8 @@
 // Whole-limb variants, degrees 2^9 .. 2^13, and the two-pass variants of
-// 2^13 (tiles of 4096 words: two CTAs of 256 threads per SM where the
-// whole-limb 2^13 tile fits one of 512; 9% faster at 512 limbs on GB300).
+// 2^13, which take every call with more limbs than the small-tile variants:
+// two CTAs of 256 threads per SM where the whole-limb 2^13 tile fits one of
+// 512 (GB300, polymul of 4096 limbs 837 against 958 us, inverse NTT 342
+// against 514).
 #include "ntt_kernels.cuh"
 
 namespace yell_gb300 {
@@ -16,6 +18,7 @@ void add_whole_variants_large(std::vector<Variant>* by) {
   by[12].push_back(whole_variant<12, 13>());
   by[13].push_back(whole_variant<13, 13>());
   by[13].push_back(two_pass_variant<13, 6>());
+  by[13].back().polymul_upto = by[13].back().ntt_upto = kAnyLimbs;
   by[13].push_back(two_pass_variant<13, 7>());
 }
 
