@@ -411,6 +411,13 @@ int yell_crt_words(uint32_t L, uint32_t cm0, uint32_t* words);
 /* d_in: count polys (count, L, N); d_out: count * N * W words. */
 int yell_dev_crt_lift(uint64_t* d_out, const uint64_t* d_in, uint32_t count, uint32_t L, uint32_t log_n,
                       uint32_t cm0, void* stream);
+/* With 4 to 32 moduli the lift's CTAs wait on the device for one another's
+ * warps, each wait for at most 1 s; one that runs out records
+ * YELL_ERR_TIMEOUT and the kernel still finishes (its output is then
+ * undefined).  This call waits for all work queued on the current device,
+ * stores the recorded status (YELL_OK or YELL_ERR_TIMEOUT) in *status and
+ * clears it. */
+int yell_crt_wait_status(uint32_t* status);
 /* Host drop-in for poly2mpz over moduli 0 .. L-1: limbs[j] -> out (N * W words). */
 int yell_poly_to_bigint(uint64_t* out, const uint64_t* const* limbs, uint32_t L, uint32_t log_n);
 

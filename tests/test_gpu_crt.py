@@ -1,10 +1,13 @@
 """GPU RNS -> big-integer lifting (gmp::poly2mpz, include/yell/gmp.hpp:42-70)
 against the big-integer oracle, word for word, plus CRT properties at full
 size and the cases that take the kernel's quotient-correction path."""
+import ctypes
+
 import numpy as np
 import pytest
 
 import yell_gb300 as y
+from yell_gb300._capi import call
 from oracle.crt import CrtTable, poly2bigint, to_words
 from yell_gb300.inputs import uniform_polys
 
@@ -109,3 +112,33 @@ def test_crt_errors(cuda):
         y.dev_crt_lift(t, t, 1, 2, 2)
     with pytest.raises(y.YellError):
         y.dev_crt_lift(t, t, 1, 2, 3, cm0=999)
+
+
+@pytest.mark.parametrize("L,log_n,cm0,count", [(3, 7, 0, 2), (4, 3, 0, 3), (4, 7, 996, 1), (5, 6, 2, 5), (8, 8, 0, 1),
+                                               (9, 7, 1, 3), (16, 4, 0, 9), (17, 7, 983, 2), (24, 6, 0, 3),
+                                               (25, 9, 0, 1), (31, 7, 969, 3), (32, 5, 968, 5), (33, 5, 0, 3)])
+def test_lift_around_the_chunk_and_kernel_edges(cuda, orc, L, log_n, cm0, count):
+    """One modulus more and less than a chunk of 8 and than the tensor-core
+    kernel takes (4 .. 32), the last primes of the table, tiles of 128
+    coefficients that are partial or span polynomials, and operands that are
+    only 8-byte aligned; residues are random or those of 0, small integers and
+    Q - k, whose quotients need the correction."""
+    ps = [orc.prime(cm0 + j) for j in range(L)]
+    t = CrtTable(ps)
+    n = 1 << log_n
+    polys = uniform_polys(L * 77 + log_n, count, L, log_n, ps)
+    special = [0, 1, 2, t.Q - 1, t.Q - 2, t.Q // 2, t.Q // 3, (1 << 64) - 1]
+    for i, x in enumerate(special[:n]):
+        polys[i % count, :, n - 1 - i] = [x % p for p in ps]
+    W = y.crt_words(L, cm0)
+    src = cuda.zeros(polys.size + 1, dtype=cuda.int64, device="cuda")
+    src[1:] = _dev(cuda, polys)
+    out = cuda.zeros(count * (W << log_n) + 1, dtype=cuda.int64, device="cuda")
+    y.dev_crt_lift(out[1:], src[1:], count, L, log_n, cm0)
+    cuda.cuda.synchronize()
+    got = out[1:].cpu().numpy().view(np.uint64).reshape(count, n, W)
+    for i in range(count):
+        assert np.array_equal(got[i], to_words(poly2bigint(polys[i], ps), W)), (L, i)
+    status = ctypes.c_uint32(1)
+    call("yell_crt_wait_status", ctypes.byref(status))
+    assert status.value == 0 and int(out[0]) == 0

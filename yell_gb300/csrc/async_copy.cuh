@@ -36,6 +36,22 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                ::"r"(d), "l"(src), "r"(bytes), "r"(b) : "memory");
 }
 
+// One try_wait: whether phase `parity` of the mbarrier has completed.  The
+// thread may be suspended for up to about 20 us first, instead of polling
+// beside the warps that it waits for.
+__device__ __forceinline__ bool mbar_test(uint64_t* mbar, uint32_t parity) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(mbar);
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 20000;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(a), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
 // Waits for phase `parity` of the mbarrier for at most timeout_ns of the
 // global timer (1 s unless given) or 2^24 polls.  When either limit runs out
 // it records `timeout_code` in *status (if still 0) and returns false.

@@ -11,7 +11,9 @@
 //         f_j = floor(y_j * floor(2^125 / q_j) / 2^61); the estimate is v or v - 1
 //   x   = sum_j y_j * (Q/q_j) - v * Q, minus Q once more when still >= Q
 // sum_j y_j * (Q/q_j) = Q * sum_j y_j / q_j, so with the exact v this is x.
-// The multi-word sums run over 32-bit digits: a thread owns one coefficient
+// With 4 to 32 moduli the sums run on the tensor cores (crt_mma.cuh).  Below
+// and above that the multi-word sums run over 32-bit digits: a thread owns one
+// coefficient
 // and keeps its y_j in shared memory; the cofactor digits are staged per tile
 // of output digits and shared by the block; x is written as W little-endian
 // words per coefficient, W = words of Q, coefficient-major.
@@ -25,6 +27,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "crt_mma.cuh"
 #include "kernels.h"
 #include "profiler.h"
 #include "runtime.h"
@@ -36,6 +39,7 @@ namespace {
 
 typedef unsigned __int128 u128;
 
+constexpr uint32_t kMmaMinModuli = 4;    // see crt_lift
 constexpr uint32_t kCrtMaxModuli = 400;  // 32 threads * 400 words * 8 B = 100 KB of y per block
 
 // Per (device, cm0, L) constants, device resident:
@@ -51,6 +55,9 @@ struct CrtTables {
   CrtConst* mods = nullptr;
   uint64_t* cofactors = nullptr;
   uint64_t* q = nullptr;
+  // the tensor-core kernel's (kMmaMinModuli <= L <= crt_mma::kMaxL)
+  crt_mma::Mod* mma_mods = nullptr;
+  uint4* image = nullptr;
 };
 
 // Host big integers: little-endian 64-bit words.
@@ -90,6 +97,87 @@ uint64_t pow_mod(uint64_t b, uint64_t e, uint64_t m) {
   return r;
 }
 
+// The first D balanced base-256 digits (-128 .. 127) of a modulo 256^D.
+std::vector<int> balanced_digits(const Big& a, uint32_t D) {
+  std::vector<int> out(D, 0);
+  int carry = 0;
+  for (uint32_t d = 0; d < D; ++d) {
+    const int byte = d / 8 < a.size() ? (int)((a[d / 8] >> (8 * (d % 8))) & 255u) : 0;
+    int v = byte + carry;
+    carry = v > 127 ? 1 : 0;
+    out[d] = v - 256 * carry;
+  }
+  return out;
+}
+
+// An integer of magnitude below 2048 * 2 as a 16-bit float (exact).
+uint16_t f16_bits(int v) {
+  if (v == 0) return 0;
+  const uint32_t sign = v < 0 ? 0x8000u : 0u;
+  uint32_t m = (uint32_t)(v < 0 ? -v : v), e = 0;
+  while ((m >> e) > 1) ++e;  // 2^e <= m
+  return (uint16_t)(sign | ((e + 15) << 10) | ((e <= 10 ? m << (10 - e) : m >> (e - 10)) & 0x3FFu));
+}
+
+// The constant matrix of the tensor-core kernel in its shared-memory layout:
+// column d, row (j, i) = digit d of (Q/q_j) * 256^i, eight moduli per chunk;
+// the tail's rows are the digits of -Q (factor v), 3072 (factor 4096) and
+// (factor 1) the digits of minus what the accumulators' offset and the bit
+// patterns' exponents add to the epilogue's sum, modulo 256^D: 2^22 at every
+// digit and 0x4B000000 at digits 0 and 2 of every four.
+std::vector<uint8_t> mma_image(uint32_t L, uint32_t W, const std::vector<uint64_t>& cof, const Big& Q) {
+  using namespace crt_mma;
+  const uint32_t N = columns(W), D = 8 * W;
+  std::vector<uint8_t> img(image_bytes(L, N), 0);
+  auto put = [&](size_t at, int v) {
+    const uint16_t h = f16_bits(v);
+    std::memcpy(img.data() + at, &h, 2);
+  };
+  for (uint32_t j = 0; j < L; ++j) {
+    const Big c(cof.begin() + (size_t)j * W, cof.begin() + (size_t)(j + 1) * W);
+    const std::vector<int> dig = balanced_digits(c, D);
+    const size_t chunk = (size_t)(j / kChunkMods) * image_chunk(N);
+    for (uint32_t i = 0; i < 8; ++i)
+      for (uint32_t d = i; d < D; ++d)
+        put(chunk + swizzle128(d * 128 + ((j % kChunkMods) * 8 + i) * 2), dig[d - i]);
+  }
+  const size_t tail = (size_t)chunks(L) * image_chunk(N);
+  Big neg(W), off(W);
+  uint64_t borrow = 0, carry = 0;
+  std::vector<uint64_t> sums(D + 8, 0);
+  for (uint32_t d = 0; d < D; ++d) {
+    sums[d + 2] += 0x40;                     // 2^22 = 0x40 * 256^2
+    if (d % 2 == 0) sums[d + 3] += 0x4B;     // 0x4B000000 = 0x4B * 256^3
+  }
+  for (uint32_t w = 0; w < W; ++w) {
+    uint64_t word = 0;
+    for (uint32_t k = 0; k < 8; ++k) {
+      carry += sums[8 * w + k];
+      word |= (carry & 255u) << (8 * k);
+      carry >>= 8;
+    }
+    off[w] = word;
+  }
+  auto negate = [&](const Big& a, Big* out) {
+    borrow = 0;
+    for (uint32_t w = 0; w < W; ++w) {
+      const uint64_t v = w < a.size() ? a[w] : 0;
+      (*out)[w] = 0 - v - borrow;
+      borrow = (v | borrow) ? 1 : 0;
+    }
+  };
+  negate(Q, &neg);
+  const std::vector<int> nq = balanced_digits(neg, D);
+  Big noff(W);
+  negate(off, &noff);
+  for (uint32_t d = 0; d < N; ++d) {
+    put(tail + swizzle32(d * 32), d < D ? nq[d] : 0);
+    put(tail + swizzle32(d * 32 + 2), 3072);
+    put(tail + swizzle32(d * 32 + 4), d < D ? (int)((noff[d / 8] >> (8 * (d % 8))) & 255u) : 0);
+  }
+  return img;
+}
+
 int build_crt_tables(uint32_t cm0, uint32_t L, CrtTables* t) {
   Big Q{1};
   for (uint32_t j = 0; j < L; ++j) big_mul_small(Q, prime_entry(cm0 + j).p);
@@ -119,10 +207,23 @@ int build_crt_tables(uint32_t cm0, uint32_t L, CrtTables* t) {
   if (e == cudaSuccess) e = cudaMemcpy(t->mods, mods.data(), L * sizeof(CrtConst), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(t->cofactors, cof.data(), cof.size() * 8, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(t->q, Q.data(), (size_t)W * 8, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && L >= kMmaMinModuli && L <= crt_mma::kMaxL) {
+    std::vector<crt_mma::Mod> mm(L);
+    for (uint32_t j = 0; j < L; ++j)
+      mm[j] = {mods[j].q, mods[j].inv, mods[j].inv_s, (int64_t)(((u128)1 << 88) / mods[j].q)};
+    const std::vector<uint8_t> img = mma_image(L, W, cof, Q);
+    e = lib_malloc(&t->mma_mods, L * sizeof(crt_mma::Mod));
+    if (e == cudaSuccess) e = lib_malloc(&t->image, img.size());
+    if (e == cudaSuccess)
+      e = cudaMemcpy(t->mma_mods, mm.data(), L * sizeof(crt_mma::Mod), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(t->image, img.data(), img.size(), cudaMemcpyHostToDevice);
+  }
   if (e != cudaSuccess) {
     cudaFree(t->mods);
     cudaFree(t->cofactors);
     cudaFree(t->q);
+    cudaFree(t->mma_mods);
+    cudaFree(t->image);
     return fail_cuda(e, "CRT tables");
   }
   t->W = W;
@@ -292,11 +393,59 @@ size_t crt_smem(uint32_t L, int threads) {
   return (size_t)L * threads * sizeof(uint64_t) + (size_t)L * (kDigitTile + 1) * sizeof(uint32_t);
 }
 
+// First status of a bounded wait of the tensor-core kernel.
+__device__ uint32_t g_crt_wait_status;
+
+cudaError_t launch_crt_mma(uint64_t* d_out, const uint64_t* d_in, uint64_t coeffs, uint32_t L, uint32_t log_n,
+                           const CrtTables* t, cudaStream_t st, int device) {
+  using namespace crt_mma;
+  static constexpr decltype(&k_crt_mma<1>) kKernels[] = {k_crt_mma<1>, k_crt_mma<2>, k_crt_mma<3>, k_crt_mma<4>};
+  static_assert(sizeof(kKernels) / sizeof(kKernels[0]) == chunks(kMaxL), "a kernel per number of chunks");
+  static std::mutex mu;
+  static std::map<int, std::pair<uint32_t, uint32_t*>> devices;  // SMs and the status word's address
+  uint32_t sms = 0;
+  uint32_t* status = nullptr;
+  {
+    std::lock_guard<std::mutex> g(mu);
+    auto it = devices.find(device);
+    if (it == devices.end()) {
+      int n = 0;
+      void* p = nullptr;
+      cudaError_t e = cudaSuccess;
+      for (auto k : kKernels)
+        if (e == cudaSuccess)
+          e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(kMaxL, 256));
+      if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
+      if (e == cudaSuccess) e = cudaGetSymbolAddress(&p, g_crt_wait_status);
+      if (e != cudaSuccess) return e;
+      it = devices.emplace(device, std::make_pair((uint32_t)n, static_cast<uint32_t*>(p))).first;
+    }
+    sms = it->second.first;
+    status = it->second.second;
+  }
+  const uint64_t tiles = (coeffs + kRows - 1) / kRows;
+  const uint32_t grid = (uint32_t)(tiles < sms ? tiles : sms);
+  LaunchScope ps("crt_lift_mma", st);
+  launch_dependent(kKernels[chunks(L) - 1], grid, kThreads, smem_bytes(L, columns(t->W)), st, d_out, d_in, coeffs, L, log_n,
+                   (const Mod*)t->mma_mods, (const uint4*)t->image, (const uint64_t*)t->q, t->W, status);
+  g_kernel_launches += 1;
+  return cudaGetLastError();
+}
+
 int crt_lift(uint64_t* d_out, const uint64_t* d_in, uint32_t count, uint32_t L, uint32_t log_n, uint32_t cm0,
              cudaStream_t st, int device) {
   const CrtTables* t = nullptr;
   int s = crt_tables(device, cm0, L, &t);
   if (s != kOk) return s;
+  // From 4 moduli up the tensor-core kernel is the faster one at every number
+  // of coefficients (GB300, us, digit kernel -> tensor cores: 2^20
+  // coefficients, L = 3: 35 -> 41, 4: 53 -> 42, 8: 117 -> 48, 16: 286 -> 80,
+  // 32: 762 -> 143; 2^13, L = 3: 6.1 -> 4.1, 32: 35 -> 6); its digits are exact
+  // up to kMaxL moduli.
+  if (t->image) {
+    const cudaError_t me = launch_crt_mma(d_out, d_in, (uint64_t)count << log_n, L, log_n, t, st, device);
+    return me == cudaSuccess ? kOk : fail_cuda(me, "crt_lift");
+  }
   // 64 threads per block while their y_j fit in 160 KB of shared memory, else 32
   // (128-thread blocks measured 2% slower at L = 32)
   const int threads = crt_smem(L, 64) <= (160u << 10) ? 64 : 32;
@@ -362,6 +511,25 @@ int yell_dev_crt_lift(uint64_t* d_out, const uint64_t* d_in, uint32_t count, uin
   if (!ctx) return st;
   return crt_lift(d_out, d_in, count, L, log_n, cm0, stream ? static_cast<cudaStream_t>(stream) : ctx->stream(),
                   ctx->device());
+}
+
+int yell_crt_wait_status(uint32_t* status) {
+  if (!status) return fail(kInvalidArgument, "null output");
+  int st = kOk;
+  DeviceContext* ctx = DeviceContext::current(&st);
+  if (!ctx) return st;
+  cudaError_t e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) return fail_cuda(e, "synchronize");
+  uint32_t v = 0;
+  e = cudaMemcpyFromSymbol(&v, g_crt_wait_status, sizeof(v));
+  if (e != cudaSuccess) return fail_cuda(e, "read wait status");
+  if (v != 0) {
+    const uint32_t zero = 0;
+    e = cudaMemcpyToSymbol(g_crt_wait_status, &zero, sizeof(zero));
+    if (e != cudaSuccess) return fail_cuda(e, "clear wait status");
+  }
+  *status = v;
+  return kOk;
 }
 
 int yell_poly_to_bigint(uint64_t* out, const uint64_t* const* limbs, uint32_t L, uint32_t log_n) {
