@@ -30,7 +30,7 @@ constexpr uint32_t kPolymulConsts = 1000;
 // Kernel launches made by this library (for the caller's accounting).
 extern std::atomic<uint64_t> g_kernel_launches;
 
-// Whether this thread's two-pass launches run as programmatic dependents of
+// Whether this thread's launches run as programmatic dependents of
 // the stream's previous kernel (their CTAs become resident during its last
 // wave and wait there).  PlainLaunches clears it for a scope whose kernels
 // share the device with other streams' work (a batch's buckets on forked
@@ -49,7 +49,8 @@ struct PlainLaunches {
 // g_dependent_launches is cleared): the kernel's CTAs may start while that
 // kernel's last CTAs finish, and wait (grid_dep_wait, common.cuh) before
 // they touch global memory other than the library's tables.  Used for the
-// two-pass NTT and polymul, the samplers and the staged 32-bit polymul.
+// NTT and polymul, the element-wise ops, the samplers, the tensor-core CRT
+// lift and the staged 32-bit polymul.
 template <typename... KArgs, typename... Args>
 void launch_dependent(void (*kernel)(KArgs...), dim3 grid, uint32_t threads, size_t smem, cudaStream_t st,
                       Args... args) {

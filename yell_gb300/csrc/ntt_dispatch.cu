@@ -30,47 +30,72 @@ __device__ __forceinline__ void st_pair(uint64_t* p, uint64_t a, uint64_t b) {
 }
 
 // ===========================================================================
-// Element-wise ops, two words per thread with 128-bit accesses.
+// Element-wise ops, a grid of up to kEwCtasPerSm CTAs per SM striding over
+// 16-byte pairs.  Bound by HBM (24 or 32 bytes per word).  addmod and submod
+// keep two pairs per operand in flight per thread; the Barrett products need
+// the registers for resident warps instead.  A grid of 8 CTAs per SM is a
+// whole and a partial wave at their occupancy (5 or 6 CTAs per SM); many
+// short CTAs level that out, while one per 256 pairs adds launch work.
+// GB300, 512 limbs of 2^16 (us, 8 CTAs per SM and one pair -> here -> one CTA
+// per 256 pairs): mulmod 138 -> 122 -> 135, muladd 156 -> 154 -> 163, addmod
+// 130 -> 118 -> 127, negate 85 -> 83 -> 96 (two pairs 88); 108 limbs of 2^15:
+// muladd 20.4 -> 18.1, addmod 16.4 -> 14.5.
 // ===========================================================================
+constexpr uint32_t kEwCtasPerSm = 24;
+constexpr bool ew_product(int op) { return op == (int)EwOp::kMulmod || op == (int)EwOp::kMuladd; }
+
 template <int OP>
 __global__ void __launch_bounds__(256) k_elementwise(LimbSet dst, ConstLimbSet a, ConstLimbSet b,
                                                      uint32_t log_n, const DevMod* __restrict__ mods) {
+  constexpr bool kBinary = OP != (int)EwOp::kNegate;
+  constexpr int kPairs = ew_product(OP) || !kBinary ? 1 : 2;
+  constexpr bool kAcc = OP == (int)EwOp::kMuladd;
+  grid_dep_launch();
+  grid_dep_wait();  // as in the two-pass kernels
   const size_t pairs = ((size_t)dst.count << log_n) >> 1;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
   const uint32_t nmask = (1u << log_n) - 1u;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < pairs;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const size_t v = i * 2;
-    const uint32_t limb = (uint32_t)(v >> log_n);
-    const uint32_t off = (uint32_t)v & nmask;
-    const uint32_t cm = dst.cm(limb);
-    const uint64_t p = __ldg(&mods[cm].p);
-    const ulonglong2 x = ld_pair(a.limb(limb, log_n) + off);
-    uint64_t* d = dst.limb(limb, log_n) + off;
-    uint64_t r0, r1;
-    if (OP == (int)EwOp::kNegate) {
-      r0 = p - x.x;
-      r1 = p - x.y;
-    } else {
-      const ulonglong2 y = ld_pair(b.limb(limb, log_n) + off);
-      if (OP == (int)EwOp::kAddmod) {
-        r0 = addmod(x.x, y.x, p);
-        r1 = addmod(x.y, y.y, p);
-      } else if (OP == (int)EwOp::kSubmod) {
-        r0 = submod(x.x, y.x, p);
-        r1 = submod(x.y, y.y, p);
-      } else {
-        const uint64_t pn = __ldg(&mods[cm].pn);
-        if (OP == (int)EwOp::kMulmod) {
-          r0 = mulmod_barrett(x.x, y.x, p, pn);
-          r1 = mulmod_barrett(x.y, y.y, p, pn);
-        } else {
-          const ulonglong2 acc = *reinterpret_cast<const ulonglong2*>(d);
-          r0 = muladd_barrett(acc.x, x.x, y.x, p, pn);
-          r1 = muladd_barrett(acc.y, x.y, y.y, p, pn);
-        }
+  for (size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i0 < pairs; i0 += kPairs * stride) {
+    ulonglong2 x[kPairs], y[kPairs], acc[kPairs];
+    uint64_t* d[kPairs];
+    uint64_t p[kPairs], pn[kPairs];
+#pragma unroll
+    for (int u = 0; u < kPairs; ++u) {
+      const size_t v = (i0 + u * stride) * 2;
+      if (i0 + u * stride < pairs) {
+        const uint32_t limb = (uint32_t)(v >> log_n), off = (uint32_t)v & nmask;
+        x[u] = ld_pair(a.limb(limb, log_n) + off);
+        if (kBinary) y[u] = ld_pair(b.limb(limb, log_n) + off);
+        d[u] = dst.limb(limb, log_n) + off;
+        if (kAcc) acc[u] = *reinterpret_cast<const ulonglong2*>(d[u]);
+        const DevMod* m = mods + dst.cm(limb);
+        p[u] = __ldg(&m->p);
+        pn[u] = __ldg(&m->pn);
       }
     }
-    st_pair(d, r0, r1);
+#pragma unroll
+    for (int u = 0; u < kPairs; ++u) {
+      if (i0 + u * stride < pairs) {
+        uint64_t r0, r1;
+        if (OP == (int)EwOp::kNegate) {
+          r0 = p[u] - x[u].x;
+          r1 = p[u] - x[u].y;
+        } else if (OP == (int)EwOp::kAddmod) {
+          r0 = addmod(x[u].x, y[u].x, p[u]);
+          r1 = addmod(x[u].y, y[u].y, p[u]);
+        } else if (OP == (int)EwOp::kSubmod) {
+          r0 = submod(x[u].x, y[u].x, p[u]);
+          r1 = submod(x[u].y, y[u].y, p[u]);
+        } else if (OP == (int)EwOp::kMulmod) {
+          r0 = mulmod_barrett(x[u].x, y[u].x, p[u], pn[u]);
+          r1 = mulmod_barrett(x[u].y, y[u].y, p[u], pn[u]);
+        } else {
+          r0 = muladd_barrett(acc[u].x, x[u].x, y[u].x, p[u], pn[u]);
+          r1 = muladd_barrett(acc[u].y, x[u].y, y[u].y, p[u], pn[u]);
+        }
+        st_pair(d[u], r0, r1);
+      }
+    }
   }
 }
 
@@ -204,15 +229,15 @@ cudaError_t launch_elementwise(EwOp op, const LimbSet& dst, const ConstLimbSet& 
   if (dst.count == 0) return cudaSuccess;
   const size_t pairs = ((size_t)dst.count << log_n) >> 1;
   const size_t want = (pairs + 255) / 256;
-  const size_t cap = (size_t)num_sms() * 8;
+  const size_t cap = (size_t)num_sms() * kEwCtasPerSm;
   const uint32_t grid = (uint32_t)(want < cap ? want : cap);
   LaunchScope ps("elementwise", st);
   switch (op) {
-    case EwOp::kMulmod: k_elementwise<0><<<grid, 256, 0, st>>>(dst, a, b, log_n, mods); break;
-    case EwOp::kAddmod: k_elementwise<1><<<grid, 256, 0, st>>>(dst, a, b, log_n, mods); break;
-    case EwOp::kSubmod: k_elementwise<2><<<grid, 256, 0, st>>>(dst, a, b, log_n, mods); break;
-    case EwOp::kMuladd: k_elementwise<3><<<grid, 256, 0, st>>>(dst, a, b, log_n, mods); break;
-    case EwOp::kNegate: k_elementwise<4><<<grid, 256, 0, st>>>(dst, a, b, log_n, mods); break;
+    case EwOp::kMulmod: launch_dependent(k_elementwise<0>, grid, 256, 0, st, dst, a, b, log_n, mods); break;
+    case EwOp::kAddmod: launch_dependent(k_elementwise<1>, grid, 256, 0, st, dst, a, b, log_n, mods); break;
+    case EwOp::kSubmod: launch_dependent(k_elementwise<2>, grid, 256, 0, st, dst, a, b, log_n, mods); break;
+    case EwOp::kMuladd: launch_dependent(k_elementwise<3>, grid, 256, 0, st, dst, a, b, log_n, mods); break;
+    case EwOp::kNegate: launch_dependent(k_elementwise<4>, grid, 256, 0, st, dst, a, b, log_n, mods); break;
   }
   g_kernel_launches += 1;
   return cudaGetLastError();

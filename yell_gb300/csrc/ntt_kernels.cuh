@@ -229,6 +229,8 @@ __global__ void __launch_bounds__(C::THREADS, C::THREADS <= 256 ? 3 : 1) k_ntt_w
   extern __shared__ __align__(16) uint64_t smem[];
   constexpr int K = C::K, NR = C::NR;
   const uint32_t log_n = K;
+  grid_dep_launch();
+  grid_dep_wait();  // as in k_col_pass
   const uint32_t tid = threadIdx.x;
   const uint32_t limb0 = blockIdx.x << (C::T - K);
   const uint32_t my_limb = limb0 + C::sub(tid);
@@ -591,6 +593,8 @@ __device__ __forceinline__ void polymul_whole_body(LimbSet c, ConstLimbSet a, Co
 template <class C>
 __global__ void __launch_bounds__(C::THREADS, C::THREADS <= 256 ? 2 : 1) k_polymul_whole(LimbSet c, ConstLimbSet a, ConstLimbSet b,
                                                               const DevMod* __restrict__ mods) {
+  grid_dep_launch();
+  grid_dep_wait();  // as in k_col_pass
   polymul_whole_body<C>(c, a, b, mods, blockIdx.x);
 }
 
@@ -936,9 +940,9 @@ cudaError_t launch_whole_ntt(const LimbSet& ls, const DevMod* mods, NttDir dir, 
   const size_t smem = tile_bytes(T);
   LaunchScope ps(dir == NttDir::kBackward ? "ntt_whole_inv" : "ntt_whole_fwd", st);
   switch (dir) {
-    case NttDir::kForward: k_ntt_whole<C, 0><<<grid, C::THREADS, smem, st>>>(ls, mods); break;
-    case NttDir::kForwardLazy: k_ntt_whole<C, 1><<<grid, C::THREADS, smem, st>>>(ls, mods); break;
-    case NttDir::kBackward: k_ntt_whole<C, 2><<<grid, C::THREADS, smem, st>>>(ls, mods); break;
+    case NttDir::kForward: launch_dependent(k_ntt_whole<C, 0>, grid, C::THREADS, smem, st, ls, mods); break;
+    case NttDir::kForwardLazy: launch_dependent(k_ntt_whole<C, 1>, grid, C::THREADS, smem, st, ls, mods); break;
+    case NttDir::kBackward: launch_dependent(k_ntt_whole<C, 2>, grid, C::THREADS, smem, st, ls, mods); break;
   }
   g_kernel_launches += 1;
   return cudaGetLastError();
@@ -952,7 +956,7 @@ cudaError_t launch_whole_polymul(const LimbSet& c, const ConstLimbSet& a, const 
   const uint32_t per = 1u << (T - LOGN);
   const uint32_t grid = (c.count + per - 1) / per;
   LaunchScope ps("polymul_whole", st);
-  k_polymul_whole<C><<<grid, C::THREADS, 2 * tile_bytes(T), st>>>(c, a, b, mods);
+  launch_dependent(k_polymul_whole<C>, grid, C::THREADS, 2 * tile_bytes(T), st, c, a, b, mods);
   g_kernel_launches += 1;
   return cudaGetLastError();
 }
