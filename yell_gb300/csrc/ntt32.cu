@@ -2,18 +2,18 @@
 // -DYELL_USE_32BITS_MODULI: include/yell/params_32.hpp, 291 30-bit primes,
 // uint32 words and uint64 products, degrees up to kMaxPolyDegree = 2^15).
 //
-// The kernels reuse the tile engine of the 64-bit path at 32-bit words.  A CTA
-// holds whole limbs in shared memory (2^T words, T = max(log_n, 11), several
-// limbs per CTA below 2^11); every word is read from HBM once and written
-// once.  The single-CTA fused polymul keeps one operand tile in shared memory
-// at a time: NTT(a) leaves its last forward round in registers and parks the
-// reduced words in the output limb (the same thread reads them back, so they
-// stay in L2), NTT(b) then runs in the same buffer, and the product, inverse
-// rounds and scaled last layer follow.  At 2^14 and 2^15 a limb is split over
-// a CTA pair whose operands arrive by bulk asynchronous copies, b's while a
-// computes, and a's NTT waits in shared memory.  The butterflies, their order
-// and their twiddle indices are the reference's, so lazy words match it
-// exactly.
+// The kernels reuse the tile engine of the 64-bit path at 32-bit words.  Up to
+// 2^13 a CTA can hold whole limbs in shared memory (2^T words, T =
+// max(log_n, 11), several limbs per CTA below 2^11); every word is read from
+// HBM once and written once.  That fused polymul keeps one operand tile in
+// shared memory at a time: NTT(a) leaves its last forward round in registers
+// and parks the reduced words in the output limb (the same thread reads them
+// back, so they stay in L2), NTT(b) then runs in the same buffer, and the
+// product, inverse rounds and scaled last layer follow.  From 2^10 up a limb
+// can also be split over a cluster (the 64-bit path's cluster kernels at
+// 32-bit words), by the number of limbs up to 2^13 and always above
+// (kCluster32).  The butterflies, their order and their twiddle indices are
+// the reference's, so lazy words match it exactly.
 #include <algorithm>
 #include <cstring>
 #include <memory>
@@ -26,6 +26,7 @@
 
 #include "async_copy.cuh"
 #include "kernels.h"
+#include "ntt_cluster.cuh"
 #include "ntt_tile.cuh"
 #include "profiler.h"
 #include "runtime.h"
@@ -344,16 +345,16 @@ __global__ void __launch_bounds__(C::THREADS, 1024 / C::THREADS) k32_polymul(uin
 }
 
 
-// ---- polymul by a CTA pair (thread-block cluster of 2) ------------------------
-// For N = 2^14 and 2^15 one limb is split over two CTAs of one cluster, each
-// holding half of it (2^(log N - 1) words, 64 KB at 2^15).  The forward stage
-// that pairs words N/2 apart (stage 0, twiddle w[1]) is applied while
-// loading: each CTA reads both halves (the second read of a word comes from
-// L2) and keeps the butterfly output of its own half.  Stages 1 .. log N - 1
-// stay inside a half (group G = the CTA's rank).  The inverse's last layer
-// (N^-1 scaling fused) pairs the halves again: after a cluster barrier each
-// CTA reads the peer's words through distributed shared memory and writes its
-// own half of the outputs.
+// ---- polymul at 2^15 by a CTA pair with staged operands ------------------------
+// One limb is split over the two CTAs of a cluster, each holding half of it.
+// The forward stage that pairs words N/2 apart (stage 0, twiddle w[1]) is
+// applied to the raw operand: each CTA brings the whole limb and keeps the
+// butterfly output of its own half.  Stages 1 .. log N - 1 stay inside a half
+// (group G = the CTA's rank).  The inverse's last layer (N^-1 scaling fused)
+// pairs the halves again: after a cluster barrier each CTA reads the peer's
+// words through distributed shared memory and writes its own half of the
+// outputs.  One CTA of 1024 threads per SM, so 76 limbs are one wave; used
+// only around that size (kCluster32).
 //
 // The stages inside a half limb of 2^H words run as two tiles of the engine:
 // the top KTOP (pair distances 2^(H-1) .. 2^(H-KTOP)) across the CTA (CA:
@@ -373,89 +374,14 @@ struct HalfSplit {
   }
 };
 
-// Geometry of a CTA-pair kernel: half limbs of 2^(LOGN-1) words, 2^LOGE words
-// per thread, the top KTOP stages of the half across the CTA.
-template <int LOGN, int LOGE_, int KTOP_>
+// Geometry: 1024-thread CTAs of 16 words per thread at 64 registers, the top 7
+// stages across the CTA and rows of 128 words (6 or 8 stages across the CTA
+// measured 0 and 2% slower, 512 threads of 32 words 2 to 15%).
 struct PairGeom32 {
-  static constexpr int H = LOGN - 1;
-  static constexpr int LOGE = LOGE_;
-  static constexpr int KTOP = KTOP_;
+  static constexpr int H = 14, LOGE = 4, KTOP = 7;
   using C = TileCfg<H, H, 0, LOGE>;
   using S = HalfSplit<H, LOGE, KTOP>;
-  static constexpr int MIN_BLOCKS = C::THREADS <= 256 ? 3 : (C::THREADS <= 512 ? 2 : 1);
-  static constexpr size_t kSmem = Smem<uint32_t>::words(1u << H) * sizeof(uint32_t);
 };
-
-// Polymul.  2^14: 256-thread CTAs of 32 words per thread, three per SM at 80
-// registers.  2^15: 1024-thread CTAs of 16 words per thread, one per SM at 64
-// registers, top 7 stages across the CTA and rows of 128 words: the same 32
-// resident warps per SM as two 512-thread CTAs of 32 words, without their
-// 216 bytes of register spills, and 1024 CTA-sized units per 512-limb launch
-// fill 6.7 waves of 152 SMs where limb pairs filled 3.4 waves of 304 slots.
-// Measured on GB300 (N = 2^15, L = 32, 16 pairs): 0.2228 ms, the same as two
-// 512-thread CTAs per SM (0.2228 ms); with the top 6 or 8 stages across the
-// CTA 0.2238 and 0.2273 ms.  Staged (k32_polymul_pair_staged, one CTA per SM
-// by its shared memory), 512-thread CTAs of 32 words at 128 registers took
-// 0.2087 / 0.2195 / 0.2353 ms with the top 5 / 6 / 7 stages across the CTA,
-// against 0.2053 ms for this geometry.
-template <int LOGN>
-using PairCfg32 = PairGeom32<LOGN, (LOGN >= 15 ? 4 : 5), (LOGN >= 15 ? 7 : 5)>;
-
-// NTT alone: 32 words per thread at both degrees; at 2^15 two 512-thread CTAs
-// per SM (64 registers, no spills) with the top 5 stages across the CTA:
-// rounds of 5 stages, one exchange fewer per transform.  Measured (2^15,
-// L = 32, 16 polys): backward 90.7 -> 77.1 us, forward 83.4 / 83.8 us.
-template <int LOGN>
-using NttPairCfg32 = PairGeom32<LOGN, 5, 5>;
-
-// Forward NTT of one half limb of `src` (the limb's first word) into the
-// bottom-round registers x of this thread: stage 0 while loading, stages
-// 1 .. log N - 1 in shared memory, the last round in registers.
-template <class PC, bool CLUSTER_SYNC = false>
-__device__ __forceinline__ void pair_forward(uint32_t* x, const uint32_t* __restrict__ src, uint32_t* smem32,
-                                             uint32_t tid, uint32_t r, const DevMod32& m, uint2 w1) {
-  using C = typename PC::C;
-  using S = typename PC::S;
-  constexpr int H = C::K, NR = C::NR;
-  constexpr uint32_t half = 1u << H;
-  constexpr int IT = (int)(half / (C::THREADS * 4));
-  constexpr int BATCH = IT < 2 ? IT : 2;  // loads in flight per thread: 2 x BATCH x 16 bytes
-  using RB = Round<C, NR - 1>;
-  const uint32_t p = m.p, p2 = p << 1, np = 0u - p;
-#pragma unroll 1  // unrolled, the loads of every batch get hoisted together and spill
-  for (int i0 = 0; i0 < IT; i0 += BATCH) {
-    uint4 lo[BATCH], hi[BATCH];
-#pragma unroll
-    for (int i = 0; i < BATCH; ++i) {
-      const uint32_t v = (tid + (i0 + i) * C::THREADS) * 4;
-      lo[i] = __ldg(reinterpret_cast<const uint4*>(src + v));
-      hi[i] = __ldg(reinterpret_cast<const uint4*>(src + half + v));
-    }
-#pragma unroll
-    for (int i = 0; i < BATCH; ++i) {
-      const uint32_t v = (tid + (i0 + i) * C::THREADS) * 4;
-      uint32_t u0[4] = {lo[i].x, lo[i].y, lo[i].z, lo[i].w}, u1[4] = {hi[i].x, hi[i].y, hi[i].z, hi[i].w};
-#pragma unroll
-      for (int k = 0; k < 4; ++k) ct_bfly(u0[k], u1[k], w1.x, w1.y, np, p2);
-      *reinterpret_cast<uint4*>(smem32 + Smem<uint32_t>::idx(v)) =
-          r == 0 ? make_uint4(u0[0], u0[1], u0[2], u0[3]) : make_uint4(u1[0], u1[1], u1[2], u1[3]);
-    }
-  }
-  // an in-place transform may overwrite src only once both CTAs have read it
-  if constexpr (CLUSTER_SYNC) cooperative_groups::this_cluster().sync();
-  else __syncthreads();
-  using CA = typename S::CA;
-  using CB = typename S::CB;
-  using RBB = Round<CB, CB::NR - 1>;
-  static_assert(RBB::R == RB::R && RBB::BETA == 0 && RBB::EB == 0, "same bottom round as one tile over the half");
-  constexpr uint32_t s_rows = 1 + S::KTOP_STAGES;  // first stage of the rows
-  fwd_rounds<CA, 0, CA::NR>(smem32, tid, 1, r, m.fwd, p, true);  // stages 1..KTOP, CTA barriers
-  const uint32_t G = S::row_group(r, tid);
-  fwd_rounds<CB, 0, CB::NR - 1, CB::LOCAL_BARRIER>(smem32, tid, s_rows, G, m.fwd, p, true);
-  const uint32_t bb = RBB::base(tid);
-  smem_load<RBB>(x, smem32, bb);
-  ct_round<RBB>(x, m.fwd, s_rows + RBB::HI, RBB::gr(bb, G), p);
-}
 
 // Inverse stages inside the half limb from the bottom-round registers x:
 // rows (warp barriers), then the top KTOP across the CTA; the words end in
@@ -503,56 +429,8 @@ __device__ __forceinline__ void pair_last_layer(uint32_t* dst, const uint32_t* s
   }
 }
 
-template <class PC>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PC::C::THREADS, PC::MIN_BLOCKS)
-    k32_polymul_pair(uint32_t* c, const uint32_t* a, const uint32_t* b, Limbs32 ls,
-                     const DevMod32* __restrict__ mods) {
-  namespace cg = cooperative_groups;
-  using C = typename PC::C;
-  extern __shared__ __align__(16) uint32_t smem32[];
-  constexpr int H = C::K, NR = C::NR, E = 1 << C::LOGE;
-  constexpr uint32_t log_n = H + 1, half = 1u << H;
-  constexpr int IT = (int)(half / (C::THREADS * 4));
-  using RB = Round<C, NR - 1>;
-  static_assert(RB::R == C::LOGE && RB::BETA == 0 && RB::EB == 0, "bottom round must own contiguous words");
-  static_assert(IT * C::THREADS * 4 == (int)half, "half limb not a whole number of 16-byte chunks per thread");
-  static_assert(IT % 2 == 0 || IT == 1, "stage-in batches of two");
-  cg::cluster_group cluster = cg::this_cluster();
-  const uint32_t r = cluster.block_rank();  // which half of the limb
-  const uint32_t limb = blockIdx.x >> 1;    // grid = 2 x limbs, every CTA active
-  const uint32_t tid = threadIdx.x;
-  const DevMod32 m = load_mod(mods, ls.cm(limb));
-  const uint32_t p = m.p, p2 = p << 1;
-  const uint2 w1 = __ldg(m.fwd + 1);
-  const size_t lbase = (size_t)limb << log_n;
-  const uint32_t bb = RB::base(tid);
-  uint32_t* park = c + lbase + r * half + bb;
-  uint32_t x[E];
-  pair_forward<PC>(x, a + lbase, smem32, tid, r, m, w1);
-#pragma unroll
-  for (int i = 0; i < E; i += 4)
-    *reinterpret_cast<uint4*>(park + i) =
-        make_uint4(csub(x[i], p2), csub(x[i + 1], p2), csub(x[i + 2], p2), csub(x[i + 3], p2));
-  __syncthreads();  // the buffer is reused for b
-  pair_forward<PC>(x, b + lbase, smem32, tid, r, m, w1);
-#pragma unroll
-  for (int i = 0; i < E; i += 4) {
-    const uint4 ah = *reinterpret_cast<const uint4*>(park + i);  // written above by this thread
-    x[i] = mont_mul(ah.x, csub(x[i], p2), p, m.pn);
-    x[i + 1] = mont_mul(ah.y, csub(x[i + 1], p2), p, m.pn);
-    x[i + 2] = mont_mul(ah.z, csub(x[i + 2], p2), p, m.pn);
-    x[i + 3] = mont_mul(ah.w, csub(x[i + 3], p2), p, m.pn);
-  }
-  pair_inverse<PC>(x, smem32, tid, r, bb, m);
-  cluster.sync();
-  pair_last_layer<PC, true>(c + lbase + r * half, smem32, cluster.map_shared_rank(smem32, (int)(r ^ 1u)), tid, r, m);
-  cluster.sync();  // the peer may still be reading this CTA's shared memory
-}
-
-// ---- polymul by a CTA pair with staged operands ------------------------------
-// The same butterflies as k32_polymul_pair, with the operands moved by bulk
-// asynchronous copies (cp.async.bulk, completion counted on an mbarrier):
-// both halves of a's limb land in a raw staging area S of shared memory; the
+// The operands move by bulk asynchronous copies (cp.async.bulk, completion
+// counted on an mbarrier): both halves of a's limb land in a raw staging area S of shared memory; the
 // stage-0 butterflies read them from there; then b's copy into S starts and
 // runs while a's remaining stages compute.  a's reduced NTT stays in the work
 // tile W where its bottom round left it, and b is transformed in place in S
@@ -619,7 +497,7 @@ __device__ __forceinline__ void stage0_from_smem(uint32_t* dst, const uint32_t* 
 }
 
 // Stages 1 .. log N - 1 of the half limb in `work` (after stage 0), the last
-// round into the registers x; the same rounds as pair_forward.
+// round into the registers x.
 template <class PC>
 __device__ __forceinline__ void pair_forward_rounds(uint32_t* x, uint32_t* work, uint32_t tid, uint32_t r,
                                                     const DevMod32& m) {
@@ -637,23 +515,16 @@ __device__ __forceinline__ void pair_forward_rounds(uint32_t* x, uint32_t* work,
   ct_round<RBB>(x, m.fwd, s_rows + RBB::HI, RBB::gr(bb, G), m.p);
 }
 
-template <int LOGN>
-struct StagedCfg32 {
-  using PC = PairCfg32<LOGN>;
-  static constexpr uint32_t kHalf = 1u << (LOGN - 1);
-  static constexpr size_t kSmem = 3 * (size_t)kHalf * sizeof(uint32_t) + 16;  // W, S, mbarrier
-  static constexpr int MIN_BLOCKS = (int)(228 * 1024 / (kSmem + 1024)) < PC::MIN_BLOCKS
-                                        ? (int)(228 * 1024 / (kSmem + 1024))
-                                        : PC::MIN_BLOCKS;
+struct Staged32 {
+  static constexpr int THREADS = PairGeom32::C::THREADS;
+  static constexpr size_t kSmem = 3 * (size_t(1) << PairGeom32::H) * sizeof(uint32_t) + 16;  // W, S, mbarrier
 };
 
-template <int LOGN>
-__global__ void __cluster_dims__(2, 1, 1)
-    __launch_bounds__(PairCfg32<LOGN>::C::THREADS, StagedCfg32<LOGN>::MIN_BLOCKS)
-    k32_polymul_pair_staged(uint32_t* c, const uint32_t* a, const uint32_t* b, Limbs32 ls,
-                            const DevMod32* __restrict__ mods) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Staged32::THREADS, 1)
+    k32_polymul_staged(uint32_t* c, const uint32_t* a, const uint32_t* b, Limbs32 ls,
+                       const DevMod32* __restrict__ mods) {
   namespace cg = cooperative_groups;
-  using PC = PairCfg32<LOGN>;
+  using PC = PairGeom32;
   using C = typename PC::C;
   extern __shared__ __align__(128) uint32_t smem_st[];
   constexpr int H = C::K, NR = C::NR, E = 1 << C::LOGE;
@@ -716,59 +587,6 @@ __global__ void __cluster_dims__(2, 1, 1)
   cluster.sync();  // the peer may still be reading this CTA's shared memory
 }
 
-// In-place NTT of one limb by a CTA pair (DIR: 0 forward, 1 forward lazy,
-// 2 backward), same split as k32_polymul_pair.
-template <class PC, int DIR>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PC::C::THREADS, PC::MIN_BLOCKS)
-    k32_ntt_pair(uint32_t* data, Limbs32 ls, const DevMod32* __restrict__ mods) {
-  namespace cg = cooperative_groups;
-  using C = typename PC::C;
-  using S = typename PC::S;
-  extern __shared__ __align__(16) uint32_t smem32[];
-  constexpr int H = C::K, NR = C::NR, E = 1 << C::LOGE;
-  constexpr uint32_t log_n = H + 1, half = 1u << H;
-  constexpr int IT = (int)(half / (C::THREADS * 4));
-  using RB = Round<C, NR - 1>;
-  cg::cluster_group cluster = cg::this_cluster();
-  const uint32_t r = cluster.block_rank();
-  const uint32_t limb = blockIdx.x >> 1;
-  const uint32_t tid = threadIdx.x;
-  const DevMod32 m = load_mod(mods, ls.cm(limb));
-  const uint32_t p = m.p, p2 = p << 1;
-  uint32_t* base = data + ((size_t)limb << log_n);
-  if constexpr (DIR != 2) {
-    uint32_t x[E];
-    pair_forward<PC, true>(x, base, smem32, tid, r, m, __ldg(m.fwd + 1));
-    uint32_t* out = base + r * half + RB::base(tid);
-#pragma unroll
-    for (int i = 0; i < E; i += 4) {
-      uint4 v = make_uint4(x[i], x[i + 1], x[i + 2], x[i + 3]);
-      if (DIR == 0) v = make_uint4(fwd_correct(v.x, p, p2), fwd_correct(v.y, p, p2), fwd_correct(v.z, p, p2),
-                                   fwd_correct(v.w, p, p2));
-      *reinterpret_cast<uint4*>(out + i) = v;
-    }
-  } else {
-    const uint32_t* own = base + r * half;
-#pragma unroll 1
-    for (int i = 0; i < IT; ++i) {
-      const uint32_t v = (tid + i * C::THREADS) * 4;
-      *reinterpret_cast<uint4*>(smem32 + Smem<uint32_t>::idx(v)) = __ldg(reinterpret_cast<const uint4*>(own + v));
-    }
-    __syncthreads();
-    {
-      using CA = typename S::CA;
-      using CB = typename S::CB;
-      const uint32_t G = S::row_group(r, tid);
-      inv_rounds<CB, CB::NR - 1, 0, false, CB::LOCAL_BARRIER>(smem32, tid, log_n, 0, G, m, true);
-      inv_rounds<CB, 0, -1, false>(smem32, tid, log_n, 0, G, m, true);  // CTA barrier after
-      inv_rounds<CA, CA::NR - 1, -1, false>(smem32, tid, log_n, S::KB, r, m, true);
-    }
-    cluster.sync();
-    pair_last_layer<PC, false>(base + r * half, smem32, cluster.map_shared_rank(smem32, (int)(r ^ 1u)), tid, r, m);
-    cluster.sync();
-  }
-}
-
 template <int OP>
 __global__ void k32_elementwise(uint32_t* dst, const uint32_t* a, const uint32_t* b, size_t total, uint32_t log_n,
                                 Limbs32 ls, const DevMod32* __restrict__ mods) {
@@ -784,14 +602,10 @@ __global__ void k32_elementwise(uint32_t* dst, const uint32_t* a, const uint32_t
 }
 
 // ---- launch ----------------------------------------------------------------------
-// Degrees whose polymul runs on a CTA pair, with staged operands
-// (k32_polymul_pair_staged; measured on GB300 at L = 32 and 2^20 words per
-// operand: 2^15 203.6 us against 223.3 us for k32_polymul_pair, 2^14 176.4
-// against 195.9 us).
-constexpr int kMinPairLogN = 14;
-constexpr int kStagedMinLogN = 14;
-// Host-pointer calls up to this degree (single-CTA kernels) run in place on
-// the context's pinned, device-mapped host buffer.
+// Degrees of the one-CTA kernels; larger ones run on clusters only.
+constexpr int kLogMaxOneCta32 = 13;
+// Host-pointer calls up to this degree run in place on the context's pinned,
+// device-mapped host buffer.
 constexpr uint32_t kSmallCall32LogN = 13;
 
 template <int LOGN>
@@ -799,20 +613,11 @@ cudaError_t set_attrs32() {
   using C = typename Cfg32<LOGN>::C;
   const int smem = (int)Cfg32<LOGN>::kSmem;
   cudaError_t e = cudaSuccess;
-  for (auto k : {k32_ntt<C, 0>, k32_ntt<C, 1>, k32_ntt<C, 2>})
+  for (auto k : {k32_ntt<C, 0>, k32_ntt<C, 1>})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k32_polymul<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if constexpr (LOGN >= kMinPairLogN) {
-    using PC = PairCfg32<LOGN>;
-    using NC = NttPairCfg32<LOGN>;
-    for (auto k : {k32_ntt_pair<NC, 0>, k32_ntt_pair<NC, 1>, k32_ntt_pair<NC, 2>})
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NC::kSmem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k32_polymul_pair<PC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)PC::kSmem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k32_polymul_pair_staged<LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)StagedCfg32<LOGN>::kSmem);
+  if constexpr (LOGN < kLogMaxOneCta32) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k32_ntt<C, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k32_polymul<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   }
   return e;
 }
@@ -823,27 +628,136 @@ cudaError_t launch32(int kind, uint32_t* c, const uint32_t* a, const uint32_t* b
   using CF = Cfg32<LOGN>;
   using C = typename CF::C;
   const uint32_t blocks = (ls.count + (1u << (C::T - LOGN)) - 1) >> (C::T - LOGN);
-  if (kind == 3) mods += kMaxModuli32;  // the fused polymul's copy of the constants
-  if constexpr (LOGN >= kMinPairLogN) {
-    using PC = PairCfg32<LOGN>;
-    using P = typename PC::C;
-    using NC = NttPairCfg32<LOGN>;
-    using NP = typename NC::C;
-    const uint32_t g = 2 * ls.count;
-    if (kind == 0) k32_ntt_pair<NC, 0><<<g, NP::THREADS, NC::kSmem, st>>>(c, ls, mods);
-    else if (kind == 1) k32_ntt_pair<NC, 1><<<g, NP::THREADS, NC::kSmem, st>>>(c, ls, mods);
-    else if (kind == 2) k32_ntt_pair<NC, 2><<<g, NP::THREADS, NC::kSmem, st>>>(c, ls, mods);
-    else if (LOGN >= kStagedMinLogN)  // a programmatic dependent of the stream's previous kernel
-      launch_dependent(k32_polymul_pair_staged<LOGN>, g, P::THREADS, StagedCfg32<LOGN>::kSmem, st, c, a, b, ls,
-                       mods);
-    else k32_polymul_pair<PC><<<g, P::THREADS, PC::kSmem, st>>>(c, a, b, ls, mods);
-    return cudaGetLastError();
-  }
   if (kind == 0) k32_ntt<C, 0><<<blocks, C::THREADS, CF::kSmem, st>>>(c, ls, mods);
   else if (kind == 1) k32_ntt<C, 1><<<blocks, C::THREADS, CF::kSmem, st>>>(c, ls, mods);
-  else if (kind == 2) k32_ntt<C, 2><<<blocks, C::THREADS, CF::kSmem, st>>>(c, ls, mods);
-  else k32_polymul<C><<<blocks, C::THREADS, CF::kSmem, st>>>(c, a, b, ls, mods);
+  if constexpr (LOGN < kLogMaxOneCta32) {  // at 2^13 clusters take every inverse and polymul
+    if (kind == 2) k32_ntt<C, 2><<<blocks, C::THREADS, CF::kSmem, st>>>(c, ls, mods);
+    else if (kind == 3) k32_polymul<C><<<blocks, C::THREADS, CF::kSmem, st>>>(c, a, b, ls, mods + kMaxModuli32);
+  }
   return cudaGetLastError();
+}
+
+// Contiguous 32-bit limbs for the cluster kernels (the interface of LimbSet).
+template <class P>
+struct LimbSet32 {
+  P* base;
+  uint32_t count, L, cm0;
+  __device__ __forceinline__ P* limb(uint32_t k, uint32_t log_n) const { return base + ((size_t)k << log_n); }
+  __device__ __forceinline__ uint32_t cm(uint32_t k) const { return cm0 + k % L; }
+  __device__ __forceinline__ uint32_t ordered(uint32_t i) const {  // modulus-major, as LimbSet
+    const uint32_t polys = count / L;
+    return (i % polys) * L + i / polys;
+  }
+};
+using Out32 = LimbSet32<uint32_t>;
+using In32 = LimbSet32<const uint32_t>;
+
+template <class CC>
+cudaError_t cluster_ntt32(int kind, uint32_t* c, const Limbs32& ls, const DevMod32* mods, cudaStream_t st) {
+  const Out32 o{c, ls.count, ls.L, ls.cm0};
+  if (kind == 0) launch_cluster<CC>(k_ntt_cluster<CC, 0, Out32, DevMod32>, ls.count, 2 * CC::kTileBytes, st, o, mods);
+  else if (kind == 1)
+    launch_cluster<CC>(k_ntt_cluster<CC, 1, Out32, DevMod32>, ls.count, 2 * CC::kTileBytes, st, o, mods);
+  else launch_cluster<CC>(k_ntt_cluster<CC, 2, Out32, DevMod32>, ls.count, 2 * CC::kTileBytes, st, o, mods);
+  return cudaGetLastError();
+}
+template <class CC>
+cudaError_t cluster_polymul32(uint32_t* c, const uint32_t* a, const uint32_t* b, const Limbs32& ls,
+                              const DevMod32* mods, cudaStream_t st) {
+  launch_cluster<CC>(k_polymul_cluster<CC, Out32, In32, DevMod32>, ls.count, 4 * CC::kTileBytes, st,
+                     Out32{c, ls.count, ls.L, ls.cm0}, In32{a, ls.count, ls.L, ls.cm0},
+                     In32{b, ls.count, ls.L, ls.cm0}, mods + kMaxModuli32);
+  return cudaGetLastError();
+}
+template <class CC>
+cudaError_t attrs_ntt32() {
+  constexpr size_t bytes = 2 * CC::kTileBytes > kSpreadBytes ? 2 * CC::kTileBytes : kSpreadBytes;
+  cudaError_t e = set_smem(k_ntt_cluster<CC, 0, Out32, DevMod32>, bytes);
+  if (e == cudaSuccess) e = set_smem(k_ntt_cluster<CC, 1, Out32, DevMod32>, bytes);
+  return e == cudaSuccess ? set_smem(k_ntt_cluster<CC, 2, Out32, DevMod32>, bytes) : e;
+}
+template <class CC>
+cudaError_t attrs_polymul32() {
+  return set_smem(k_polymul_cluster<CC, Out32, In32, DevMod32>,
+                  4 * CC::kTileBytes > kSpreadBytes ? 4 * CC::kTileBytes : kSpreadBytes);
+}
+cudaError_t staged_polymul32(uint32_t* c, const uint32_t* a, const uint32_t* b, const Limbs32& ls,
+                             const DevMod32* mods, cudaStream_t st) {
+  launch_dependent(k32_polymul_staged, 2 * ls.count, Staged32::THREADS, Staged32::kSmem, st, c, a, b, ls,
+                   mods + kMaxModuli32);
+  return cudaGetLastError();
+}
+cudaError_t attrs_staged32() { return set_smem(k32_polymul_staged, Staged32::kSmem); }
+
+// Cluster kernels (one limb per cluster of 2^CL CTAs) by degree and number of
+// limbs: a call takes the entry of its degree with the smallest bound that
+// its limbs do not exceed, else the one-CTA kernels above (2^3 .. 2^13).  The
+// polymul shares every twiddle load between its operands, where the one-CTA
+// kernels transform one after the other; with few limbs a limb spread over
+// 2, 4 or 8 SMs is a shorter chain.  Past the bounds the one-CTA kernels win,
+// which exchange nothing between CTAs.  The last template argument is the
+// CTAs per SM that the polymul is compiled for: registers against residency.
+//
+// GB300, us (one-CTA and CTA-pair kernels -> here), polymul / forward /
+// inverse: 8 limbs of 2^13 16.5 -> 6.0 / 8.2 -> 5.3 / 8.2 -> 5.4; 24 of 2^14
+// 21.3 -> 9.5 / 10.3 -> 7.5 / 12.3 -> 7.3; 512 of 2^13 51.2 -> 40.2 / 19.6 ->
+// 18.6 / 20.7 -> 17.1; 512 of 2^14 90.8 -> 84.9 / 39.2 -> 35.0 / 39.2 -> 32.5;
+// 512 of 2^15 200 -> 188 / 82 -> 72 / 76 -> 66.  At the bounds: 1024 limbs of
+// 2^11 polymul 20.6 -> 19.8 (1536: 28.9 against 32.7), 1536 of 2^12 61.2 -> 59.3
+// (2048: 77.1 against 79.4), 768 of 2^13 forward 27.1 -> 26.8 (1536: 45.7
+// against 47.8).  57 to 76 limbs of 2^15 are one wave of the staged CTA pair
+// (28 us), but two of the three clusters' worth of SMs that 8 CTAs each need
+// (32 to 34 us).
+struct Cluster32 {
+  uint32_t log_n;
+  uint32_t polymul_upto, fwd_upto, inv_upto;  // 0: never
+  cudaError_t (*ntt)(int, uint32_t*, const Limbs32&, const DevMod32*, cudaStream_t);
+  cudaError_t (*polymul)(uint32_t*, const uint32_t*, const uint32_t*, const Limbs32&, const DevMod32*, cudaStream_t);
+  cudaError_t (*ntt_attrs)();
+  cudaError_t (*polymul_attrs)();
+};
+template <int LOGN, int K1, int LOGE, int CL, int PB = 0>
+using CC32 = ClusterCfg<LOGN, K1, LOGE, CL, uint32_t, PB>;
+template <class CC>
+constexpr Cluster32 polymul_route32(uint32_t upto) {
+  return {CC::LOGN, upto, 0, 0, nullptr, cluster_polymul32<CC>, nullptr, attrs_polymul32<CC>};
+}
+template <class CC>
+constexpr Cluster32 ntt_route32(uint32_t fwd, uint32_t inv) {
+  return {CC::LOGN, 0, fwd, inv, cluster_ntt32<CC>, nullptr, attrs_ntt32<CC>, nullptr};
+}
+constexpr uint32_t kAny32 = 0xFFFFFFFFu;
+constexpr Cluster32 kCluster32[] = {
+    polymul_route32<CC32<10, 5, 3, 1>>(1024),
+    ntt_route32<CC32<10, 5, 3, 1>>(1024, 1024),
+    polymul_route32<CC32<11, 5, 3, 1>>(1024),
+    ntt_route32<CC32<11, 5, 3, 1>>(768, 512),
+    polymul_route32<CC32<12, 6, 3, 1>>(224),
+    polymul_route32<CC32<12, 6, 4, 1, 4>>(1536),
+    ntt_route32<CC32<12, 6, 3, 2>>(288, 288),
+    ntt_route32<CC32<12, 6, 3, 1>>(1536, 768),
+    polymul_route32<CC32<13, 6, 3, 2>>(100),
+    polymul_route32<CC32<13, 6, 4, 1, 3>>(kAny32),
+    ntt_route32<CC32<13, 6, 3, 2>>(400, 400),
+    ntt_route32<CC32<13, 6, 4, 1>>(768, kAny32),
+    polymul_route32<CC32<14, 7, 4, 2, 2>>(76),
+    polymul_route32<CC32<14, 7, 4, 2, 3>>(kAny32),
+    ntt_route32<CC32<14, 7, 4, 3>>(200, 200),
+    ntt_route32<CC32<14, 7, 4, 2>>(kAny32, kAny32),
+    polymul_route32<CC32<15, 8, 4, 3, 2>>(32),
+    polymul_route32<CC32<15, 8, 4, 3, 3>>(57),
+    {15, 76, 0, 0, nullptr, staged_polymul32, nullptr, attrs_staged32},
+    polymul_route32<CC32<15, 8, 4, 3, 3>>(kAny32),
+    ntt_route32<CC32<15, 8, 4, 3>>(kAny32, kAny32),
+};
+
+// The entry of kCluster32 for a call, or nullptr.
+const Cluster32* route32(uint32_t log_n, int kind, uint32_t limbs) {
+  const auto bound = kind == 3 ? &Cluster32::polymul_upto : (kind == 2 ? &Cluster32::inv_upto : &Cluster32::fwd_upto);
+  const Cluster32* best = nullptr;
+  for (const Cluster32& r : kCluster32)
+    if (r.log_n == log_n && r.*bound >= limbs && (!best || r.*bound < best->*bound)) best = &r;
+  return best;
 }
 
 template <int... L>
@@ -861,7 +775,8 @@ cudaError_t attrs32(std::integer_sequence<int, L...>) {
   return e;
 }
 
-using Degrees32 = std::make_integer_sequence<int, kLogMaxDegree32 - kMinLogN32 + 1>;
+// The degrees of the one-CTA kernels.
+using OneCta32 = std::make_integer_sequence<int, kLogMaxOneCta32 - kMinLogN32 + 1>;
 
 int prepare32(uint32_t log_n, uint32_t cm0, uint32_t L, DeviceContext** ctx, const DevMod32** mods) {
   if (log_n < kMinLogN32 || log_n > kLogMaxDegree32)
@@ -877,7 +792,11 @@ int prepare32(uint32_t log_n, uint32_t cm0, uint32_t L, DeviceContext** ctx, con
     std::lock_guard<std::mutex> g(mu);
     const int dev = (*ctx)->device();
     if (std::find(done.begin(), done.end(), dev) == done.end()) {
-      const cudaError_t e = attrs32(Degrees32{});
+      cudaError_t e = attrs32(OneCta32{});
+      for (const Cluster32& r : kCluster32) {
+        if (e == cudaSuccess && r.ntt_attrs) e = r.ntt_attrs();
+        if (e == cudaSuccess && r.polymul_attrs) e = r.polymul_attrs();
+      }
       if (e != cudaSuccess) return fail_cuda(e, "32-bit kernel attributes");
       done.push_back(dev);
     }
@@ -905,7 +824,10 @@ int run32(int kind, uint32_t* c, const uint32_t* a, const uint32_t* b, uint32_t 
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->stream();
   static const char* names[4] = {"ntt32_forward", "ntt32_forward_lazy", "ntt32_backward", "polymul32"};
   LaunchScope ps(names[kind], s);
-  const cudaError_t e = dispatch32(Degrees32{}, log_n, kind, c, a, b, ls, mods, s);
+  const Cluster32* r = route32(log_n, kind, ls.count);
+  const cudaError_t e = !r ? dispatch32(OneCta32{}, log_n, kind, c, a, b, ls, mods, s)
+                        : kind == 3 ? r->polymul(c, a, b, ls, mods, s)
+                                    : r->ntt(kind, c, ls, mods, s);
   g_kernel_launches += 1;
   return e == cudaSuccess ? kOk : fail_cuda(e, names[kind]);
 }

@@ -39,12 +39,20 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t smem_addr, uint32_t rank) 
 __device__ __forceinline__ void st_cluster(uint32_t addr, uint64_t v) {
   asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
 }
+__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void st_cluster2(uint32_t addr, uint32_t v0, uint32_t v1) {
+  asm volatile("st.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(v0), "r"(v1) : "memory");
+}
 __device__ __forceinline__ void st_cluster2(uint32_t addr, uint64_t v0, uint64_t v1) {
   asm volatile("st.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(addr), "l"(v0), "l"(v1) : "memory");
 }
 
-template <int LOGN_, int K1_, int LOGE_, int CL_>
+template <int LOGN_, int K1_, int LOGE_, int CL_, class W_ = uint64_t, int PB_ = 0>
 struct ClusterCfg {
+  static constexpr int kPolymulBlocks = PB_;  // CTAs per SM that the polymul is compiled for (0: any)
+  using W = W_;
   static constexpr int LOGN = LOGN_, K1 = K1_, LOGE = LOGE_, CL = CL_;
   static constexpr int LOGB = LOGN - K1;  // words per row
   static constexpr int T = LOGN - CL;     // words per CTA
@@ -52,14 +60,15 @@ struct ClusterCfg {
   using Col = TileCfg<T, K1, LB, LOGE>;
   using Row = TileCfg<T, LOGB, 0, LOGE>;
   static constexpr int THREADS = Col::THREADS;
-  static constexpr size_t kTileBytes = tile_smem_words(1u << T) * sizeof(uint64_t);
+  static constexpr uint32_t kTileWords = Smem<W>::words(1u << T);
+  static constexpr size_t kTileBytes = kTileWords * sizeof(W);
   static_assert(LB >= 1 && K1 >= CL, "every CTA owns whole columns and whole rows");
 };
 
 // Words of column round RG, at tile indices base_v + off (row c of the limb =
 // index >> LB), to the CTAs that own their rows.  dst: the receiving tile.
-template <class CC, class RG>
-__device__ __forceinline__ void send_to_rows(const uint64_t* x, const uint64_t* dst, uint32_t base_v, uint32_t rank) {
+template <class CC, class RG, class W>
+__device__ __forceinline__ void send_to_rows(const W* x, const W* dst, uint32_t base_v, uint32_t rank) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
 #pragma unroll
   for (int ex = 0; ex < RG::E; ++ex)
@@ -68,19 +77,19 @@ __device__ __forceinline__ void send_to_rows(const uint64_t* x, const uint64_t* 
       const uint32_t v = base_v + RG::off(ex, j);
       const uint32_t c = v >> CC::LB, col = (rank << CC::LB) | (v & ((1u << CC::LB) - 1u));
       const uint32_t u = ((c & ((1u << (CC::K1 - CC::CL)) - 1u)) << CC::LOGB) | col;
-      st_cluster(map_rank(d + 8 * sidx(u), c >> (CC::K1 - CC::CL)), x[(ex << RG::R) | j]);
+      st_cluster(map_rank(d + (uint32_t)sizeof(W) * Smem<W>::idx(u), c >> (CC::K1 - CC::CL)), x[(ex << RG::R) | j]);
     }
 }
 
 // Words of row round RG, at tile indices base_v + off (column = index mod
 // 2^LOGB), to the CTAs that own their columns.
-template <class CC, class RG>
-__device__ __forceinline__ void send_to_cols(const uint64_t* x, const uint64_t* dst, uint32_t base_v, uint32_t rank) {
+template <class CC, class RG, class W>
+__device__ __forceinline__ void send_to_cols(const W* x, const W* dst, uint32_t base_v, uint32_t rank) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   auto address = [&](uint32_t u) {
     const uint32_t col = u & ((1u << CC::LOGB) - 1u);
     const uint32_t c = (rank << (CC::K1 - CC::CL)) | (u >> CC::LOGB);
-    return map_rank(d + 8 * sidx((c << CC::LB) | (col & ((1u << CC::LB) - 1u))), col >> CC::LB);
+    return map_rank(d + (uint32_t)sizeof(W) * Smem<W>::idx((c << CC::LB) | (col & ((1u << CC::LB) - 1u))), col >> CC::LB);
   };
   if constexpr (RG::PAIRS) {  // adjacent columns of one CTA (LB >= 1)
 #pragma unroll
@@ -100,32 +109,34 @@ __device__ __forceinline__ void send_to_cols(const uint64_t* x, const uint64_t* 
 // DIR: 0 forward (reduced), 1 forward lazy, 2 backward.  In place: every CTA
 // of the cluster has its words in registers or shared memory before the
 // cluster barrier, and stores only after it.
-template <class CC, int DIR>
-__global__ void __launch_bounds__(CC::THREADS) k_ntt_cluster(LimbSet ls, const DevMod* __restrict__ mods) {
-  extern __shared__ __align__(16) uint64_t smem[];
+template <class CC, int DIR, class LS, class M>
+__global__ void __launch_bounds__(CC::THREADS) k_ntt_cluster(LS ls, const M* __restrict__ mods) {
+  extern __shared__ __align__(16) uint64_t smem_c[];
+  using W = typename CC::W;
+  W* smem = reinterpret_cast<W*>(smem_c);
   using Col = typename CC::Col;
   using Row = typename CC::Row;
   constexpr uint32_t log_n = CC::LOGN;
   constexpr int E = 1 << CC::LOGE;
-  uint64_t* sc = smem;                                 // column tile
-  uint64_t* sr = smem + tile_smem_words(1u << CC::T);  // row tile
+  W* sc = smem;                   // column tile
+  W* sr = smem + CC::kTileWords;  // row tile
   cluster_arrive();  // the peers have started: awaited before the first word is sent
   grid_dep_launch();
   grid_dep_wait();  // as in k_col_pass
   const uint32_t tid = threadIdx.x;
   const uint32_t rank = blockIdx.x & ((1u << CC::CL) - 1u);  // of a one-dimensional cluster
   const uint32_t limb = ls.ordered(blockIdx.x >> CC::CL);
-  uint64_t* data = ls.limb(limb, log_n);
-  const DevMod m = load_mod(mods, ls.cm(limb));
+  W* data = ls.limb(limb, log_n);
+  const M m = load_mod(mods, ls.cm(limb));
   const uint32_t G = (rank << (CC::K1 - CC::CL)) + Row::sub(tid);
-  uint64_t x[E];
+  W x[E];
   using C0 = Round<Col, 0>;
   using CL_ = Round<Col, Col::NR - 1>;
   using R0 = Round<Row, 0>;
   using RL = Round<Row, Row::NR - 1>;
   const uint32_t c0 = C0::base(tid), cl = CL_::base(tid), r0 = R0::base(tid), rl = RL::base(tid);
   if constexpr (DIR != 2) {
-    gload_cols<C0, CC::LOGB>(x, data + (rank << CC::LB), c0);
+    gload_cols<C0, CC::LOGB>(x, (const W*)data + (rank << CC::LB), c0);
     ct_round<C0>(x, m.fwd, C0::HI, C0::gr(c0, 0), m.p);
     if constexpr (Col::NR > 1) {
       smem_store<C0>(x, sc, c0);
@@ -143,11 +154,11 @@ __global__ void __launch_bounds__(CC::THREADS) k_ntt_cluster(LimbSet ls, const D
     ct_round<RL>(x, m.fwd, CC::K1 + RL::HI, RL::gr(rl, G), m.p);
     if constexpr (DIR == 0) {
 #pragma unroll
-      for (int i = 0; i < E; ++i) x[i] = fwd_correct(x[i], m.p, m.p << 1);
+      for (int i = 0; i < E; ++i) x[i] = fwd_correct(x[i], m.p, (W)(m.p << 1));
     }
     gstore_rows<RL>(x, data + ((size_t)rank << CC::T), rl);
   } else {
-    gload_rows<RL>(x, data + ((size_t)rank << CC::T), rl);
+    gload_rows<RL>(x, (const W*)data + ((size_t)rank << CC::T), rl);
     gs_round<RL, false>(x, log_n, RL::BETA, RL::gr(rl, G), m);
     if constexpr (Row::NR > 1) {
       smem_store<RL>(x, sr, rl);
@@ -168,28 +179,30 @@ __global__ void __launch_bounds__(CC::THREADS) k_ntt_cluster(LimbSet ls, const D
 }
 
 // c = INTT(NTT(a) * NTT(b)) per limb, without scratch.
-template <class CC>
-__global__ void __launch_bounds__(CC::THREADS)
-    k_polymul_cluster(LimbSet c, ConstLimbSet a, ConstLimbSet b, const DevMod* __restrict__ mods) {
-  extern __shared__ __align__(16) uint64_t smem[];
+template <class CC, class LS, class CLS, class M>
+__global__ void __launch_bounds__(CC::THREADS, CC::kPolymulBlocks)
+    k_polymul_cluster(LS c, CLS a, CLS b, const M* __restrict__ mods) {
+  extern __shared__ __align__(16) uint64_t smem_c[];
+  using W = typename CC::W;
+  W* smem = reinterpret_cast<W*>(smem_c);
   using Col = typename CC::Col;
   using Row = typename CC::Row;
   constexpr uint32_t log_n = CC::LOGN;
   constexpr int E = 1 << CC::LOGE;
-  constexpr uint32_t W = tile_smem_words(1u << CC::T);
+  constexpr uint32_t TW = CC::kTileWords;
   constexpr int BK = Row::LOCAL_BARRIER;
-  uint64_t *sa = smem, *sb = smem + W;                // column tiles
-  uint64_t *ra = smem + 2 * W, *rb = smem + 3 * W;    // row tiles
+  W *sa = smem, *sb = smem + TW;              // column tiles
+  W *ra = smem + 2 * TW, *rb = smem + 3 * TW;  // row tiles
   cluster_arrive();
   grid_dep_launch();
   grid_dep_wait();  // as in k_col_pass
   const uint32_t tid = threadIdx.x;
   const uint32_t rank = blockIdx.x & ((1u << CC::CL) - 1u);
   const uint32_t limb = c.ordered(blockIdx.x >> CC::CL);
-  const DevMod m = load_mod(mods, c.cm(limb));
-  const uint64_t np = 0 - m.p, p2 = m.p << 1;
+  const M m = load_mod(mods, c.cm(limb));
+  const W np = (W)(0 - m.p), p2 = (W)(m.p << 1);
   const uint32_t G = (rank << (CC::K1 - CC::CL)) + Row::sub(tid);
-  uint64_t xa[E], xb[E];
+  W xa[E], xb[E];
   using C0 = Round<Col, 0>;
   using CL_ = Round<Col, Col::NR - 1>;
   using R0 = Round<Row, 0>;
@@ -211,7 +224,7 @@ __global__ void __launch_bounds__(CC::THREADS)
   send_to_rows<CC, CL_>(xa, ra, cl, rank);
   send_to_rows<CC, CL_>(xb, rb, cl, rank);
   cluster_arrive();
-  const ulonglong2 w0 = fused_w0<Row>(rb0, CC::K1, G, m);
+  const auto w0 = fused_w0<Row>(rb0, CC::K1, G, m);
   cluster_wait();
   fwd_rounds2<Row, 0, Row::NR - 1, BK>(ra, rb, tid, CC::K1, G, m.fwd, m.p, true);
   smem_load<RB>(xa, ra, rb0);
@@ -289,11 +302,11 @@ template <class CC>
 cudaError_t launch_cluster_ntt(const LimbSet& ls, const DevMod* mods, NttDir dir, cudaStream_t st) {
   LaunchScope ps(dir == NttDir::kBackward ? "ntt_cluster_inv" : "ntt_cluster_fwd", st);
   switch (dir) {
-    case NttDir::kForward: launch_cluster<CC>(k_ntt_cluster<CC, 0>, ls.count, 2 * CC::kTileBytes, st, ls, mods); break;
+    case NttDir::kForward: launch_cluster<CC>(k_ntt_cluster<CC, 0, LimbSet, DevMod>, ls.count, 2 * CC::kTileBytes, st, ls, mods); break;
     case NttDir::kForwardLazy:
-      launch_cluster<CC>(k_ntt_cluster<CC, 1>, ls.count, 2 * CC::kTileBytes, st, ls, mods);
+      launch_cluster<CC>(k_ntt_cluster<CC, 1, LimbSet, DevMod>, ls.count, 2 * CC::kTileBytes, st, ls, mods);
       break;
-    case NttDir::kBackward: launch_cluster<CC>(k_ntt_cluster<CC, 2>, ls.count, 2 * CC::kTileBytes, st, ls, mods); break;
+    case NttDir::kBackward: launch_cluster<CC>(k_ntt_cluster<CC, 2, LimbSet, DevMod>, ls.count, 2 * CC::kTileBytes, st, ls, mods); break;
   }
   g_kernel_launches += 1;
   return cudaGetLastError();
@@ -304,7 +317,7 @@ cudaError_t launch_cluster_polymul(const LimbSet& c, const ConstLimbSet& a, cons
                                    uint64_t*, uint64_t* const*, cudaStream_t st) {
   mods += kPolymulConsts;  // the fused polymul's copy of the constants
   LaunchScope ps("polymul_cluster", st);
-  launch_cluster<CC>(k_polymul_cluster<CC>, c.count, 4 * CC::kTileBytes, st, c, a, b, mods);
+  launch_cluster<CC>(k_polymul_cluster<CC, LimbSet, ConstLimbSet, DevMod>, c.count, 4 * CC::kTileBytes, st, c, a, b, mods);
   g_kernel_launches += 1;
   return cudaGetLastError();
 }
@@ -314,10 +327,10 @@ cudaError_t set_attrs_cluster() {
   constexpr size_t ntt = 2 * CC::kTileBytes > kSpreadBytes ? 2 * CC::kTileBytes : kSpreadBytes;
   constexpr size_t polymul = 4 * CC::kTileBytes > kSpreadBytes ? 4 * CC::kTileBytes : kSpreadBytes;
   cudaError_t e;
-  if ((e = set_smem(k_ntt_cluster<CC, 0>, ntt)) != cudaSuccess) return e;
-  if ((e = set_smem(k_ntt_cluster<CC, 1>, ntt)) != cudaSuccess) return e;
-  if ((e = set_smem(k_ntt_cluster<CC, 2>, ntt)) != cudaSuccess) return e;
-  return set_smem(k_polymul_cluster<CC>, polymul);
+  if ((e = set_smem(k_ntt_cluster<CC, 0, LimbSet, DevMod>, ntt)) != cudaSuccess) return e;
+  if ((e = set_smem(k_ntt_cluster<CC, 1, LimbSet, DevMod>, ntt)) != cudaSuccess) return e;
+  if ((e = set_smem(k_ntt_cluster<CC, 2, LimbSet, DevMod>, ntt)) != cudaSuccess) return e;
+  return set_smem(k_polymul_cluster<CC, LimbSet, ConstLimbSet, DevMod>, polymul);
 }
 
 template <int LOGN, int K1, int LOGE, int CL>

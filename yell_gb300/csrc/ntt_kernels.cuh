@@ -60,6 +60,17 @@ __device__ __forceinline__ ulonglong2 ld_pair_t(const uint64_t* p) {
   if constexpr (COH) return ld_pair_cg(p);
   else return ld_pair(p);
 }
+// 32-bit words (only the kernels without COH use them)
+template <bool COH>
+__device__ __forceinline__ uint2 ld_pair_t(const uint32_t* p) {
+  static_assert(!COH, "32-bit words are read through the read-only path");
+  return __ldg(reinterpret_cast<const uint2*>(p));
+}
+template <bool COH>
+__device__ __forceinline__ uint32_t ld_word_t(const uint32_t* p) {
+  static_assert(!COH, "32-bit words are read through the read-only path");
+  return __ldg(p);
+}
 template <bool COH>
 __device__ __forceinline__ uint64_t ld_word_t(const uint64_t* p) {
   if constexpr (COH) return ld_cg(p);
@@ -69,27 +80,39 @@ __device__ __forceinline__ uint64_t ld_word_t(const uint64_t* p) {
 __device__ __forceinline__ void st_pair(uint64_t* p, uint64_t a, uint64_t b) {
   *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(a, b);
 }
+__device__ __forceinline__ void st_pair(uint32_t* p, uint32_t a, uint32_t b) {
+  *reinterpret_cast<uint2*>(p) = make_uint2(a, b);
+}
 
 // ---- direct global access for one round ---------------------------------------
 // Row-type region: word u of the region at g[u]; base_u and offsets are
 // u-space (tile bits below LB + K, LB = 0).
-template <class RG, bool COH = false>
-__device__ __forceinline__ void gload_rows(uint64_t* x, const uint64_t* g, uint32_t base_u) {
+template <class RG, bool COH = false, class W>
+__device__ __forceinline__ void gload_rows(W* x, const W* g, uint32_t base_u) {
   constexpr int R = RG::R;
-  const uint64_t* gb = g + base_u;
+  const W* gb = g + base_u;
   if constexpr (RG::PAIRS) {
 #pragma unroll
     for (int m = 0; m < RG::E / 2; ++m)
 #pragma unroll
       for (int j = 0; j < (1 << R); ++j) {
-        const ulonglong2 v = ld_pair_t<COH>(gb + RG::off(2 * m, j));
+        const auto v = ld_pair_t<COH>(gb + RG::off(2 * m, j));
         x[((2 * m) << R) | j] = v.x;
         x[((2 * m + 1) << R) | j] = v.y;
       }
+  } else if constexpr (RG::CONTIG && sizeof(W) == 4 && R >= 2) {
+#pragma unroll
+    for (int j = 0; j < (1 << R); j += 4) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(gb + j));
+      x[j] = v.x;
+      x[j + 1] = v.y;
+      x[j + 2] = v.z;
+      x[j + 3] = v.w;
+    }
   } else if constexpr (RG::CONTIG) {
 #pragma unroll
     for (int j = 0; j < (1 << R); j += 2) {
-      const ulonglong2 v = ld_pair_t<COH>(gb + j);
+      const auto v = ld_pair_t<COH>(gb + j);
       x[j] = v.x;
       x[j + 1] = v.y;
     }
@@ -101,16 +124,20 @@ __device__ __forceinline__ void gload_rows(uint64_t* x, const uint64_t* g, uint3
   }
 }
 
-template <class RG>
-__device__ __forceinline__ void gstore_rows(const uint64_t* x, uint64_t* g, uint32_t base_u) {
+template <class RG, class W>
+__device__ __forceinline__ void gstore_rows(const W* x, W* g, uint32_t base_u) {
   constexpr int R = RG::R;
-  uint64_t* gb = g + base_u;
+  W* gb = g + base_u;
   if constexpr (RG::PAIRS) {
 #pragma unroll
     for (int m = 0; m < RG::E / 2; ++m)
 #pragma unroll
       for (int j = 0; j < (1 << R); ++j)
         st_pair(gb + RG::off(2 * m, j), x[((2 * m) << R) | j], x[((2 * m + 1) << R) | j]);
+  } else if constexpr (RG::CONTIG && sizeof(W) == 4 && R >= 2) {
+#pragma unroll
+    for (int j = 0; j < (1 << R); j += 4)
+      *reinterpret_cast<uint4*>(gb + j) = make_uint4(x[j], x[j + 1], x[j + 2], x[j + 3]);
   } else if constexpr (RG::CONTIG) {
 #pragma unroll
     for (int j = 0; j < (1 << R); j += 2) st_pair(gb + j, x[j], x[j + 1]);
@@ -129,10 +156,10 @@ __device__ __forceinline__ size_t col_base(uint32_t base_v) {
   return ((size_t)(base_v >> RG::LB) << LOGB) + (base_v & ((1u << RG::LB) - 1u));
 }
 
-template <class RG, int LOGB, bool COH = false>
-__device__ __forceinline__ void gload_cols(uint64_t* x, const uint64_t* g, uint32_t base_v) {
+template <class RG, int LOGB, bool COH = false, class W>
+__device__ __forceinline__ void gload_cols(W* x, const W* g, uint32_t base_v) {
   constexpr int R = RG::R;
-  const uint64_t* gb = g + col_base<RG, LOGB>(base_v);
+  const W* gb = g + col_base<RG, LOGB>(base_v);
 #pragma unroll
   for (int ex = 0; ex < RG::E; ++ex)
 #pragma unroll
@@ -140,10 +167,10 @@ __device__ __forceinline__ void gload_cols(uint64_t* x, const uint64_t* g, uint3
       x[(ex << R) | j] = ld_word_t<COH>(gb + ((size_t)(RG::off(ex, j) >> RG::LB) << LOGB));
 }
 
-template <class RG, int LOGB>
-__device__ __forceinline__ void gstore_cols(const uint64_t* x, uint64_t* g, uint32_t base_v) {
+template <class RG, int LOGB, class W>
+__device__ __forceinline__ void gstore_cols(const W* x, W* g, uint32_t base_v) {
   constexpr int R = RG::R;
-  uint64_t* gb = g + col_base<RG, LOGB>(base_v);
+  W* gb = g + col_base<RG, LOGB>(base_v);
 #pragma unroll
   for (int ex = 0; ex < RG::E; ++ex)
 #pragma unroll
@@ -498,23 +525,23 @@ __global__ void __launch_bounds__(C::THREADS) k_row_pass(LimbSet ls, const DevMo
 // ===========================================================================
 // First twiddle of the fused product round (its forward top sub-stage), for
 // callers that request it a round ahead.
-template <class C>
-__device__ __forceinline__ ulonglong2 fused_w0(uint32_t b, uint32_t s_off, uint32_t G, const DevMod& m) {
+template <class C, class M>
+__device__ __forceinline__ auto fused_w0(uint32_t b, uint32_t s_off, uint32_t G, const M& m) {
   using RB = Round<C, C::NR - 1>;
   return __ldg(m.fwd + (1u << (s_off + RB::HI)) + RB::gr(b, G));
 }
 
-template <class C, bool INV_LAST>
-__device__ __forceinline__ void fused_product(uint64_t* xa, uint64_t* xb, uint32_t b, uint32_t log_n,
-                                              uint32_t s_off, uint32_t G, const DevMod& m, ulonglong2 w0) {
+template <class C, bool INV_LAST, class W, class M, class PW>
+__device__ __forceinline__ void fused_product(W* xa, W* xb, uint32_t b, uint32_t log_n, uint32_t s_off, uint32_t G,
+                                              const M& m, PW w0) {
   using RB = Round<C, C::NR - 1>;
   static_assert(RB::R == C::LOGE && RB::BETA == 0, "bottom round must be full width");
   constexpr int E = 1 << C::LOGE;
-  const uint64_t p = m.p, p2 = m.p << 1;
+  const W p = m.p, p2 = m.p << 1;
   const uint32_t gr = RB::gr(b, G);
-  ct_stages2p<RB::R, RB::E, 0>(xa, xb, m.fwd, s_off + RB::HI, gr, 0 - p, p2, &w0);
+  ct_stages2p<RB::R, RB::E, 0>(xa, xb, m.fwd, s_off + RB::HI, gr, (W)(0 - p), p2, &w0);
   // the inverse round's first twiddles load while the products compute
-  ulonglong2 wg[GsFirst<RB, INV_LAST>::N0];
+  PW wg[GsFirst<RB, INV_LAST>::N0];
   GsFirst<RB, INV_LAST>::load(wg, m.inv, log_n, 0, gr);
   // m is the polymul copy of the constants: m.pn = -p^-1 mod 2^64
 #pragma unroll

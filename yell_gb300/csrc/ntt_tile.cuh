@@ -119,9 +119,9 @@ struct Round {
 
 // ---- register <-> shared memory ----------------------------------------------
 // A 32-bit round whose thread owns 2^R consecutive words starting at a
-// multiple of 16 (the bottom round of a row tile).
+// multiple of 2^R >= 4 (the bottom round of a row tile).
 template <class RG, class W>
-constexpr bool kContig32 = sizeof(W) == 4 && RG::EB == 0 && RG::BETA == 0 && RG::LB == 0 && RG::R >= 4;
+constexpr bool kContig32 = sizeof(W) == 4 && RG::EB == 0 && RG::BETA == 0 && RG::LB == 0 && RG::R >= 2;
 
 template <class RG, class W>
 __device__ __forceinline__ void smem_load(W* x, const W* s, uint32_t base_v) {
@@ -129,7 +129,7 @@ __device__ __forceinline__ void smem_load(W* x, const W* s, uint32_t base_v) {
   using PW = typename PairOf<W>::type;
   using SL = Smem<W>;
   if constexpr (kContig32<RG, W>) {
-    // base_v has no bits below 2^R (R >= 4): idx(base_v + j) = idx(base_v) ^ j
+    // base_v has no bits below 2^R, and 4 <= 2^R <= 32: idx(base_v + j) = idx(base_v) ^ j
     const uint32_t ib = SL::idx(base_v);
 #pragma unroll
     for (int j = 0; j < (1 << R); j += 4) {

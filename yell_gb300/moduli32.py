@@ -91,7 +91,7 @@ def dev_polymul(c, a, b, pairs: int, L: int, log_n: int, cm0: int = 0, stream=No
 
 def wait_status() -> int:
     """Waits for the device's queued work and returns (and clears) the status the
-    2^14 / 2^15 polymul kernels record when a wait for their operand copies runs out."""
+    staged 2^15 polymul kernel records when a wait for its operand copies runs out."""
     import ctypes
     st = ctypes.c_uint32(0)
     call("yell32_wait_status", ctypes.byref(st))
