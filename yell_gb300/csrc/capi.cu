@@ -345,10 +345,17 @@ int yell_polymul_host(uint64_t* c, const uint64_t* a, const uint64_t* b, uint32_
     std::memcpy(c, ctx->small.host + 2 * w, w * 8);
     return kOk;
   }
-  // ~64 MiB of operands per chunk, at least one pair.
+  // ~64 MiB of operands per chunk, at least one pair.  The last chunks are
+  // smaller, so that the compute and the D2H left after the final H2D cover
+  // little, but not below 4 MiB per operand: a chunk's eleven calls take the
+  // host about 25 us, in which the link moves 5 MiB.  (GB300, 5 pairs of 8 x
+  // 2^15 words, 2 MiB each: one pair per chunk 230 us, two 182, of which the
+  // operands' transfer is 99; 8 pairs of 8 x 2^16, 4 MiB each: 499 and 498.)
   const size_t target = (64ull << 20) / 8;
   uint32_t cp = (uint32_t)std::max<size_t>(1, target / (2 * pair_words));
   if (cp > pairs) cp = pairs;
+  const size_t least = (4ull << 20) / 8;
+  const uint32_t unit = std::min<uint32_t>(cp, (uint32_t)((least + pair_words - 1) / pair_words));
   const size_t cw = cp * pair_words;
   const size_t sw = polymul_scratch_words(cp * L, log_n, ctx->shape);
   std::lock_guard<std::mutex> g(ctx->pipe_lock);
@@ -373,9 +380,8 @@ int yell_polymul_host(uint64_t* c, const uint64_t* a, const uint64_t* b, uint32_
   for (uint32_t p0 = 0, np = 0; p0 < pairs; p0 += np, ++k) {
     const int s = (int)(k % DeviceContext::kPipeSlots);
     const bool reuse = k >= (uint32_t)DeviceContext::kPipeSlots;
-    // the last cp pairs go one at a time: the compute and D2H left after the
-    // final H2D (the pipeline's tail) then cover one pair, not cp
-    np = pairs - p0 > cp ? cp : 1;
+    // the last cp pairs go `unit` at a time
+    np = pairs - p0 > cp ? cp : std::min(unit, pairs - p0);
     const size_t w = np * pair_words;
     uint64_t* da = ctx->pipe_buf[s].ptr;
     uint64_t* db = da + cw;
