@@ -512,6 +512,65 @@ __global__ void __launch_bounds__(C::THREADS) k_row_pass(LimbSet ls, const DevMo
   }
 }
 
+// The row pass of two polynomials at the same limb in one CTA: a row has as
+// many twiddles as words, twice its bytes, and they serve both.  One polynomial
+// at a time the pass waits on those loads (issue slots 34-45% used, two L2
+// sectors of twiddles per sector of words); two at a time with 8 words of each
+// per thread, tiles of 2^9 words (inverse 2^8) and 896 (1024) threads per SM
+// it is nearer the multiplier's bound.  GB300, one -> two polynomials at a
+// time, 512 limbs: 2^14 at k1 = 7 forward 49.9 -> 45.2 us, inverse 51.0 ->
+// 44.3; 2^15 100 -> 94, 112 -> 93; 2^16 207 -> 195, 233 -> 197 (inverse tiles
+// of 2^10 compiled for 768: 259).  CTAs are ordered by modulus; of an odd
+// number of polynomials the last is its own partner (its words are computed
+// and stored twice, by the same thread).
+template <class C, int K1, bool INV>
+__global__ void __launch_bounds__(C::THREADS, min_blocks(INV ? 1024 : 896, C::THREADS))
+    k_row_pass2(LimbSet ls, const DevMod* __restrict__ mods, uint32_t polys, int reduce) {
+  extern __shared__ __align__(16) uint64_t smem[];
+  constexpr int K = C::K, NR = C::NR;
+  constexpr uint32_t log_n = K + K1;
+  constexpr int TPL = log_n - C::T;
+  grid_dep_launch();
+  grid_dep_wait();  // as in k_col_pass
+  uint64_t* sa = smem;
+  uint64_t* sb = smem + tile_smem_words(1u << C::T);
+  const uint32_t tid = threadIdx.x;
+  const uint32_t unit = blockIdx.x >> TPL, half = (polys + 1) >> 1;
+  const uint32_t l = unit / half, i0 = 2 * (unit - l * half), i1 = min(i0 + 1, polys - 1);
+  const uint32_t off = (blockIdx.x & ((1u << TPL) - 1u)) << C::T;
+  uint64_t* pa = ls.limb(i0 * ls.L + l, log_n) + off;
+  uint64_t* pb = ls.limb(i1 * ls.L + l, log_n) + off;
+  const DevMod m = load_mod(mods, ls.cm0 + l);
+  const uint32_t G = (off >> K) + C::sub(tid);
+  constexpr int BK = C::LOCAL_BARRIER;
+  constexpr int E = 1 << C::LOGE;
+  uint64_t xa[E], xb[E];
+  using R0 = Round<C, 0>;
+  const uint32_t b0 = R0::base(tid);
+  if constexpr (!INV) {
+    gload_rows<R0>(xa, pa, b0);
+    gload_rows<R0>(xb, pb, b0);
+    ct_stages2<R0::R, R0::E>(xa, xb, m.fwd, K1 + R0::HI, R0::gr(b0, G), 0 - m.p, m.p << 1);
+    smem_store<R0>(xa, sa, b0);
+    smem_store<R0>(xb, sb, b0);
+    round_barrier<C, BK>(tid);
+    fwd_rounds2<C, 1, NR - 1, BK>(sa, sb, tid, K1, G, m.fwd, m.p, true);
+    fwd_rounds2<C, NR - 1, NR>(sa, sb, tid, K1, G, m.fwd, m.p, true);
+    stage_out_region<C>(sa, pa, m.p, reduce != 0);
+    stage_out_region<C>(sb, pb, m.p, reduce != 0);
+  } else {
+    stage_in_region<C>(sa, pa);
+    stage_in_region<C>(sb, pb);
+    __syncthreads();
+    inv_rounds2<C, NR - 1, 0, BK>(sa, sb, tid, log_n, 0, G, m);
+    smem_load<R0>(xa, sa, b0);
+    smem_load<R0>(xb, sb, b0);
+    gs_round2<R0>(xa, xb, log_n, R0::BETA, R0::gr(b0, G), m);
+    gstore_rows<R0>(xa, pa, b0);
+    gstore_rows<R0>(xb, pb, b0);
+  }
+}
+
 // ===========================================================================
 // Fused product round shared by both polymul kernels: the bottom forward
 // round (R = LOGE at bit 0) of both operands with shared twiddles, the
@@ -674,8 +733,8 @@ __device__ __forceinline__ void col_pass2_body(ConstLimbSet a, ConstLimbSet b, L
 template <class C>
 constexpr int two_operand_threads() { return C::LOGE == 4 ? 512 : 768; }
 
-template <class C, int LOGB>
-__global__ void __launch_bounds__(C::THREADS, min_blocks(two_operand_threads<C>(), C::THREADS))
+template <class C, int LOGB, int SM_THREADS>
+__global__ void __launch_bounds__(C::THREADS, min_blocks(SM_THREADS, C::THREADS))
     k_col_pass2(ConstLimbSet a, ConstLimbSet b, LimbSet ca, LimbSet cb, const DevMod* __restrict__ mods) {
   grid_dep_launch();
   grid_dep_wait();  // as in k_col_pass
@@ -1006,23 +1065,31 @@ cudaError_t set_attrs_whole() {
 // loads overlap more other CTAs' arithmetic) and more sectors per word in the
 // column passes; fewer words per thread more exchanges.  GB300, 512 limbs of
 // 2^16 at k1 = 7, tiles of 2^12 with 16 words per thread -> the tile below:
-// forward column pass 156 -> 147 us, forward row pass 225 -> 206, inverse row
-// pass 276 -> 233, inverse column pass 173 -> 163 (polymul 170 -> 160); 512
-// limbs of 2^14: polymul's forward column pass 87 -> 80.  Only the fused row
-// step (16 words of two operands per thread) wants its 2^12 tile: 566 us
-// against 580 at 8 words per thread and 680 at 2^10 and 2^11 words.
+// forward column pass 156 -> 144 us (147 at 2^11 words, which k1 = 6 and 8
+// prefer: 138 and 160 against 141 and 162), forward row pass 225 -> 206,
+// inverse row pass 276 -> 233, inverse column pass 173 -> 163 (polymul 170 ->
+// 160), polymul's forward column pass 291 -> 284 (8 words, compiled for 1024
+// threads per SM; 286 for 896, 296 for 768; at k1 = 6 290 -> 250); 512 limbs
+// of 2^14: 87 -> 78.  2^13 keeps 768 threads (64 limbs: 10.1 us against 11.1).
+// Only the fused row step (16 words of two operands per thread) wants its 2^12
+// tile: 566 us against 584 at 8 words per thread in tiles of 2^9 and 667 or
+// more in tiles of 2^10, compiled for 768 to 1024 threads.  RowFwd2 and RowInv2
+// are those of two polynomials at a time (k_row_pass2).
 constexpr int tile_log(int want, int least) { return want > least ? want : least; }
 
 template <int LOGN, int K1>
 struct TwoPassTiles {
   static constexpr int K = LOGN - K1;
   // the column tiles keep at least 2^2 columns (32-byte sectors)
-  using Col2 = ColCfg<LOGN, K1, (LOGN <= 15 ? 3 : 4), (LOGN <= 15 ? tile_log(10, K1 + 2) : kTileLog)>;
+  using Col2 = ColCfg<LOGN, K1, 3, tile_log(10, K1 + 2)>;
   using Rows = RowCfg<LOGN, K1>;
-  using ColFwd = ColCfg<LOGN, K1, 4, tile_log(11, K1 + 2)>;
-  using ColInv = ColFwd;
+  using ColFwd = ColCfg<LOGN, K1, 4, tile_log(K1 == 7 ? 10 : 11, K1 + 2)>;
+  using ColInv = ColCfg<LOGN, K1, 4, tile_log(11, K1 + 2)>;
   using RowFwd = RowCfg<LOGN, K1, 4, tile_log(10, K)>;
   using RowInv = RowCfg<LOGN, K1, (K <= 8 ? 3 : 4), tile_log(10, K)>;
+  using RowFwd2 = RowCfg<LOGN, K1, 3, tile_log(9, K)>;
+  using RowInv2 = RowCfg<LOGN, K1, 3, tile_log(8, K)>;
+  static constexpr int kCol2Threads = LOGN >= 14 ? 1024 : two_operand_threads<Col2>();
 };
 
 // The same tile log and words per thread for every kernel: 2^12-word tiles
@@ -1035,10 +1102,43 @@ struct UniformTiles {
   using Rows = RowCfg<LOGN, K1, LR, T>;
   using RowFwd = Rows;
   using RowInv = Rows;
+  using RowFwd2 = void;  // one polynomial at a time
+  using RowInv2 = void;
+  static constexpr int kCol2Threads = two_operand_threads<Col2>();
 };
 
 template <class C>
 constexpr size_t cfg_bytes() { return tile_bytes(C::T); }
+
+// The number of polynomials if a row pass takes them two at a time
+// (k_row_pass2), else 0.  Only for contiguous whole polynomials, whose limbs
+// of one modulus are known without reading a list.  Not for few odd ones (the
+// last is computed twice), not for forward rows of 2^11 words and more (512
+// threads per tile: 2^20 at k1 = 8, 16 limbs, 149 us one at a time, 166 two),
+// and not for inverse calls below 2^21 words, where two limbs per thread leave
+// threads missing (2^14, 64 limbs: 12.3 and 13.8 us; 2^16, 32 limbs: 22.5 and
+// 20.1).
+template <int K, bool INV>
+uint32_t paired_polys(const LimbSet& ls, uint32_t log_n) {
+  if (ls.ptrs || ls.cms || ls.L == 0 || ls.count % ls.L != 0) return 0;
+  const uint32_t polys = ls.count / ls.L;
+  if (polys < 2 || (polys % 2 != 0 && polys < 17)) return 0;
+  if (INV ? ((uint64_t)ls.count << log_n) < (1u << 21) : K > 10) return 0;
+  return polys;
+}
+
+template <class RC, class RC2, int LOGN, int K1, bool INV>
+void launch_row_pass(const LimbSet& ls, const DevMod* mods, int reduce, cudaStream_t st) {
+  if constexpr (!std::is_void_v<RC2>) {
+    if (const uint32_t polys = paired_polys<LOGN - K1, INV>(ls, LOGN)) {
+      launch_dependent(k_row_pass2<RC2, K1, INV>, (ls.L * ((polys + 1) / 2)) << (LOGN - RC2::T), RC2::THREADS,
+                       2 * cfg_bytes<RC2>(), st, ls, mods, polys, reduce);
+      return;
+    }
+  }
+  launch_dependent(k_row_pass<RC, K1, INV>, ls.count << (LOGN - RC::T), RC::THREADS, cfg_bytes<RC>(), st, ls, mods,
+                   reduce);
+}
 
 template <int LOGN, int K1, class TT>
 cudaError_t launch_two_pass_ntt(const LimbSet& ls, const DevMod* mods, NttDir dir, cudaStream_t st) {
@@ -1049,8 +1149,7 @@ cudaError_t launch_two_pass_ntt(const LimbSet& ls, const DevMod* mods, NttDir di
     using CC = typename TT::ColInv;
     {
       LaunchScope ps("row_pass_inv", st);
-      launch_dependent(k_row_pass<RC, K1, true>, ls.count << (LOGN - RC::T), RC::THREADS, cfg_bytes<RC>(), st, ls, mods,
-                       0);
+      launch_row_pass<RC, typename TT::RowInv2, LOGN, K1, true>(ls, mods, 0, st);
     }
     LaunchScope ps("col_pass_inv", st);
     launch_dependent(k_col_pass<CC, LOGB, true>, ls.count << (LOGN - CC::T), CC::THREADS, cfg_bytes<CC>(), st, cls, ls,
@@ -1064,8 +1163,7 @@ cudaError_t launch_two_pass_ntt(const LimbSet& ls, const DevMod* mods, NttDir di
                        ls, mods);
     }
     LaunchScope ps("row_pass_fwd", st);
-    launch_dependent(k_row_pass<RC, K1, false>, ls.count << (LOGN - RC::T), RC::THREADS, cfg_bytes<RC>(), st, ls, mods,
-                     dir == NttDir::kForward ? 1 : 0);
+    launch_row_pass<RC, typename TT::RowFwd2, LOGN, K1, false>(ls, mods, dir == NttDir::kForward ? 1 : 0, st);
   }
   g_kernel_launches += 2;
   return cudaGetLastError();
@@ -1085,7 +1183,7 @@ cudaError_t launch_two_pass_polymul(const LimbSet& c, const ConstLimbSet& a, con
   sl.ptrs = scratch_ptrs;
   {
     LaunchScope ps("polymul_col_fwd", st);
-    launch_dependent(k_col_pass2<C2, LOGB>, c.count << (LOGN - C2::T), C2::THREADS, 2 * cfg_bytes<C2>(), st, a, b, c,
+    launch_dependent(k_col_pass2<C2, LOGB, TT::kCol2Threads>, c.count << (LOGN - C2::T), C2::THREADS, 2 * cfg_bytes<C2>(), st, a, b, c,
                      sl, mods);
   }
   {
@@ -1114,7 +1212,15 @@ cudaError_t set_attrs_two_pass() {
     return e;
   if ((e = set_smem(k_row_pass<typename TT::RowInv, K1, true>, cfg_bytes<typename TT::RowInv>())) != cudaSuccess)
     return e;
-  if ((e = set_smem(k_col_pass2<typename TT::Col2, LOGB>, 2 * cfg_bytes<typename TT::Col2>())) != cudaSuccess) return e;
+  if constexpr (!std::is_void_v<typename TT::RowFwd2>) {
+    using F2 = typename TT::RowFwd2;
+    using I2 = typename TT::RowInv2;
+    if ((e = set_smem(k_row_pass2<F2, K1, false>, 2 * cfg_bytes<F2>())) != cudaSuccess) return e;
+    if ((e = set_smem(k_row_pass2<I2, K1, true>, 2 * cfg_bytes<I2>())) != cudaSuccess) return e;
+  }
+  if ((e = set_smem(k_col_pass2<typename TT::Col2, LOGB, TT::kCol2Threads>, 2 * cfg_bytes<typename TT::Col2>())) !=
+      cudaSuccess)
+    return e;
   return set_smem(k_polymul_rows<typename TT::Rows, K1>, 2 * cfg_bytes<typename TT::Rows>());
 }
 

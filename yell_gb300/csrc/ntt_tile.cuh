@@ -314,9 +314,11 @@ __device__ __forceinline__ void ct_stages2(W* x, W* y, const PW* __restrict__ tw
 // LAST, the round's final sub-stage is the reference's last layer with the
 // N^-1 scaling fused (include/yell/details/ntt.hpp:144-159).
 // top = log_n - 1 - sigma_first, so sub-stage k uses m = 2^(top - k).
-template <int R, int E, bool LAST, int k, class W, class PW, class M>
-__device__ __forceinline__ void gs_stages(W* x, const PW* __restrict__ itw, uint32_t top, uint32_t gr,
+// With OPS = 2, y is a second operand at the same positions.
+template <int R, int E, bool LAST, int k, int OPS, class W, class PW, class M>
+__device__ __forceinline__ void gs_stages(W* x, W* y, const PW* __restrict__ itw, uint32_t top, uint32_t gr,
                                           const M& m, const PW* wk) {
+  static_assert(OPS == 1 || !LAST, "two operands: row passes only");
   if constexpr (k < R) {
     constexpr int d = 1 << k;
     if constexpr (LAST && k == R - 1) {
@@ -341,8 +343,9 @@ __device__ __forceinline__ void gs_stages(W* x, const PW* __restrict__ itw, uint
           for (int q = 0; q < d; ++q) {
             const int j = jj * 2 * d + q;
             gs_bfly(x[(ex << R) | j], x[(ex << R) | (j + d)], wk[jj].x, wk[jj].y, np, p2);
+            if constexpr (OPS == 2) gs_bfly(y[(ex << R) | j], y[(ex << R) | (j + d)], wk[jj].x, wk[jj].y, np, p2);
           }
-      gs_stages<R, E, LAST, k + 1>(x, itw, top, gr, m, wn);
+      gs_stages<R, E, LAST, k + 1, OPS>(x, y, itw, top, gr, m, wn);
     }
   }
 }
@@ -366,7 +369,7 @@ struct GsFirst {
 template <class RG, bool LAST, class W, class M, class PW>
 __device__ __forceinline__ void gs_round_w(W* x, uint32_t log_n, uint32_t sigma_first, uint32_t gr, const M& m,
                                            const PW* w0) {
-  gs_stages<RG::R, RG::E, LAST, 0>(x, m.inv, log_n - 1 - sigma_first, gr, m, w0);
+  gs_stages<RG::R, RG::E, LAST, 0, 1>(x, x, m.inv, log_n - 1 - sigma_first, gr, m, w0);
 }
 
 template <class RG, bool LAST, class W, class M>
@@ -375,6 +378,13 @@ __device__ __forceinline__ void gs_round(W* x, uint32_t log_n, uint32_t sigma_fi
   PW w0[GsFirst<RG, LAST>::N0];
   GsFirst<RG, LAST>::load(w0, m.inv, log_n, sigma_first, gr);
   gs_round_w<RG, LAST>(x, log_n, sigma_first, gr, m, w0);
+}
+
+template <class RG, class W, class M>
+__device__ __forceinline__ void gs_round2(W* x, W* y, uint32_t log_n, uint32_t sigma_first, uint32_t gr, const M& m) {
+  typename PairOf<W>::type w0[GsFirst<RG, false>::N0];
+  GsFirst<RG, false>::load(w0, m.inv, log_n, sigma_first, gr);
+  gs_stages<RG::R, RG::E, false, 0, 2>(x, y, m.inv, log_n - 1 - sigma_first, gr, m, w0);
 }
 
 // Reads the DevMod for modulus index cm with read-only loads.
@@ -496,6 +506,25 @@ __device__ __forceinline__ void inv_rounds(W* s, uint32_t tid, uint32_t log_n, u
     inv_round_smem<C, I, HAS_LAST && I == 0>(s, tid, log_n, sig_off, G, m, active);
     round_barrier<C, BK>(tid);
     inv_rounds<C, I - 1, I1, HAS_LAST, BK>(s, tid, log_n, sig_off, G, m, active);
+  }
+}
+
+// Inverse rounds [I, I1) of two operands at the same positions, bottom-up, a
+// barrier after each.
+template <class C, int I, int I1, int BK = 0, class W, class M>
+__device__ __forceinline__ void inv_rounds2(W* sa, W* sb, uint32_t tid, uint32_t log_n, uint32_t sig_off, uint32_t G,
+                                            const M& m) {
+  if constexpr (I > I1) {
+    using RG = Round<C, I>;
+    W xa[1 << C::LOGE], xb[1 << C::LOGE];
+    const uint32_t b = RG::base(tid);
+    smem_load<RG>(xa, sa, b);
+    smem_load<RG>(xb, sb, b);
+    gs_round2<RG>(xa, xb, log_n, sig_off + RG::BETA, RG::gr(b, G), m);
+    smem_store<RG>(xa, sa, b);
+    smem_store<RG>(xb, sb, b);
+    round_barrier<C, BK>(tid);
+    inv_rounds2<C, I - 1, I1, BK>(sa, sb, tid, log_n, sig_off, G, m);
   }
 }
 
