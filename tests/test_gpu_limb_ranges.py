@@ -1,0 +1,25 @@
+"""The ranges of limbs that a variant for few limbs is chosen for: on both
+sides of every end, as in test_gpu_few_limbs (whose counts cover the ranges'
+upper ends beyond these)."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from test_gpu_few_limbs import SCRIPT
+
+pytestmark = pytest.mark.gpu
+
+COUNTS = {10: [80, 81, 160, 161, 1024, 1025], 12: [48, 49],
+          13: [15, 16, 19, 20, 33, 34, 39, 40, 48, 49, 52, 53, 56], 14: [11, 12, 22, 23, 28, 29, 36, 37],
+          15: [4, 5, 11, 12, 14, 15], 16: [2, 3, 7, 10, 11], 17: [2, 3, 5]}
+
+
+@pytest.mark.parametrize("log_n", sorted(COUNTS))
+def test_both_sides_of_the_ranges(cuda, orc, log_n):
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = {k: v for k, v in os.environ.items() if k != "YELL_GB300_TUNE_FILE"}
+    r = subprocess.run([sys.executable, "-c", SCRIPT % (log_n, COUNTS[log_n])], cwd=root, env=env,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "few limbs ok" in r.stdout, r.stdout[-500:] + r.stderr[-1500:]

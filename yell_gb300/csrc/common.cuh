@@ -345,8 +345,14 @@ template <> struct PairOf<uint32_t> {
 // visible (at once for a kernel launched without the attribute, or when the
 // stream's previous work is not a kernel), and every such kernel calls it
 // before it reads or writes global memory other than the library's own
-// tables.  grid_dep_launch() at the start of a CTA lets the stream's next
-// kernel begin launching once every CTA of this one has started.
+// tables.  grid_dep_launch() lets the stream's next kernel begin launching
+// once every CTA of this one has called it.  The transforms and polymuls call
+// it after grid_dep_wait(), so that only one kernel's CTAs wait at a time:
+// called before it, a chain of small kernels filled the SMs with waiting CTAs
+// and the running kernel's were packed onto what was left (GB300, polymul of 2
+// limbs of 2^15: 15.9 us with the launch before the wait, 10.7 after; 1 of
+// 2^16 17.2 and 10.6; NTT of 3 limbs of 2^16 9.5 and 7.5).  In the samplers and
+// the element-wise ops the order made no difference; they call it first.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -543,8 +543,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Staged32::THREADS, 1
   const uint2 w1 = __ldg(m.fwd + 1);
   const size_t lbase = (size_t)limb << log_n;
   const uint32_t bb = RB::base(tid);
-  grid_dep_launch();
   grid_dep_wait();  // the stream's previous kernel may produce a or b, or read c
+  grid_dep_launch();
   if (tid == 0) {
     mbar_init(mbar, 1);
     mbar_expect(mbar, 2 * half * (uint32_t)sizeof(uint32_t));
@@ -671,15 +671,14 @@ cudaError_t cluster_polymul32(uint32_t* c, const uint32_t* a, const uint32_t* b,
 }
 template <class CC>
 cudaError_t attrs_ntt32() {
-  constexpr size_t bytes = 2 * CC::kTileBytes > kSpreadBytes ? 2 * CC::kTileBytes : kSpreadBytes;
+  constexpr size_t bytes = 2 * CC::kTileBytes;
   cudaError_t e = set_smem(k_ntt_cluster<CC, 0, Out32, DevMod32>, bytes);
   if (e == cudaSuccess) e = set_smem(k_ntt_cluster<CC, 1, Out32, DevMod32>, bytes);
   return e == cudaSuccess ? set_smem(k_ntt_cluster<CC, 2, Out32, DevMod32>, bytes) : e;
 }
 template <class CC>
 cudaError_t attrs_polymul32() {
-  return set_smem(k_polymul_cluster<CC, Out32, In32, DevMod32>,
-                  4 * CC::kTileBytes > kSpreadBytes ? 4 * CC::kTileBytes : kSpreadBytes);
+  return set_smem(k_polymul_cluster<CC, Out32, In32, DevMod32>, 4 * CC::kTileBytes);
 }
 cudaError_t staged_polymul32(uint32_t* c, const uint32_t* a, const uint32_t* b, const Limbs32& ls,
                              const DevMod32* mods, cudaStream_t st) {

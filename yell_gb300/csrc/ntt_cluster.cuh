@@ -121,8 +121,8 @@ __global__ void __launch_bounds__(CC::THREADS) k_ntt_cluster(LS ls, const M* __r
   W* sc = smem;                   // column tile
   W* sr = smem + CC::kTileWords;  // row tile
   cluster_arrive();  // the peers have started: awaited before the first word is sent
-  grid_dep_launch();
   grid_dep_wait();  // as in k_col_pass
+  grid_dep_launch();
   const uint32_t tid = threadIdx.x;
   const uint32_t rank = blockIdx.x & ((1u << CC::CL) - 1u);  // of a one-dimensional cluster
   const uint32_t limb = ls.ordered(blockIdx.x >> CC::CL);
@@ -194,8 +194,8 @@ __global__ void __launch_bounds__(CC::THREADS, CC::kPolymulBlocks)
   W *sa = smem, *sb = smem + TW;              // column tiles
   W *ra = smem + 2 * TW, *rb = smem + 3 * TW;  // row tiles
   cluster_arrive();
-  grid_dep_launch();
   grid_dep_wait();  // as in k_col_pass
+  grid_dep_launch();
   const uint32_t tid = threadIdx.x;
   const uint32_t rank = blockIdx.x & ((1u << CC::CL) - 1u);
   const uint32_t limb = c.ordered(blockIdx.x >> CC::CL);
@@ -247,36 +247,8 @@ __global__ void __launch_bounds__(CC::THREADS, CC::kPolymulBlocks)
   gstore_cols<C0, CC::LOGB>(xa, c.limb(limb, log_n) + (rank << CC::LB), c0);
 }
 
-// Shared memory that leaves room for one CTA per SM: the scheduler otherwise
-// places several CTAs of a cluster on one SM while others stay idle.
-constexpr size_t kSpreadBytes = 116 << 10;
-
-// Clusters that are resident at once on the current device with one CTA per
-// SM, asked once per device.
-template <class CC, typename KernelT>
-uint32_t spread_clusters(KernelT kernel, cudaLaunchConfig_t cfg) {
-  static std::atomic<uint32_t> cached[64];  // the number + 1
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  uint32_t n = cached[dev].load(std::memory_order_relaxed);
-  if (n == 0) {
-    int clusters = 0;
-    cfg.dynamicSmemBytes = kSpreadBytes;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) {
-      (void)cudaGetLastError();
-      clusters = 0;
-    }
-    n = (uint32_t)clusters + 1;
-    cached[dev].store(n, std::memory_order_relaxed);
-  }
-  return n - 1;
-}
-
 // Launch of a cluster kernel, as a programmatic dependent like the two-pass
-// kernels.  When all clusters are resident at once with one CTA per SM, the
-// launch asks for that (GB300, 12 limbs of 2^13: polymul 11.6 -> 8.6 us; 8
-// of 2^14: 22.4 -> 13.9), except where other streams' kernels share the SMs.
+// kernels.
 template <class CC, typename... KArgs, typename... Args>
 void launch_cluster(void (*kernel)(KArgs...), uint32_t limbs, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchAttribute attr[2];
@@ -293,8 +265,6 @@ void launch_cluster(void (*kernel)(KArgs...), uint32_t limbs, size_t smem, cudaS
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = g_dependent_launches ? 2 : 1;
-  if (g_dependent_launches && smem < kSpreadBytes && limbs <= spread_clusters<CC>(kernel, cfg))
-    cfg.dynamicSmemBytes = kSpreadBytes;
   (void)cudaLaunchKernelEx(&cfg, kernel, args...);  // errors surface through cudaGetLastError
 }
 
@@ -324,8 +294,7 @@ cudaError_t launch_cluster_polymul(const LimbSet& c, const ConstLimbSet& a, cons
 
 template <class CC>
 cudaError_t set_attrs_cluster() {
-  constexpr size_t ntt = 2 * CC::kTileBytes > kSpreadBytes ? 2 * CC::kTileBytes : kSpreadBytes;
-  constexpr size_t polymul = 4 * CC::kTileBytes > kSpreadBytes ? 4 * CC::kTileBytes : kSpreadBytes;
+  constexpr size_t ntt = 2 * CC::kTileBytes, polymul = 4 * CC::kTileBytes;
   cudaError_t e;
   if ((e = set_smem(k_ntt_cluster<CC, 0, LimbSet, DevMod>, ntt)) != cudaSuccess) return e;
   if ((e = set_smem(k_ntt_cluster<CC, 1, LimbSet, DevMod>, ntt)) != cudaSuccess) return e;

@@ -138,13 +138,18 @@ int current_device() {
 
 // The variant a call of `limbs` limbs runs: the selected one, else the one
 // registered for that many limbs, else the first.
-const Variant& pick(uint32_t log_n, uint32_t limbs, uint32_t Variant::*bound) {
+const Variant& pick(uint32_t log_n, uint32_t limbs, LimbRange (Variant::*ranges)[2]) {
   const std::vector<Variant>& vs = variants_of(log_n);
   const uint32_t sel = g_selected[current_device()][log_n].load(std::memory_order_relaxed);
   if (sel != 0 && sel <= vs.size()) return vs[sel - 1];
   const Variant* best = &vs[0];
+  uint64_t most = ~0ull;
   for (const Variant& v : vs)
-    if (v.*bound >= limbs && (best->*bound < limbs || v.*bound < best->*bound)) best = &v;
+    for (const LimbRange& r : v.*ranges)
+      if (r.least <= limbs && limbs <= r.most && r.most < most) {
+        best = &v;
+        most = r.most;
+      }
   return *best;
 }
 
@@ -201,7 +206,7 @@ cudaError_t launch_ntt(const LimbSet& ls, uint32_t log_n, const DevMod* mods, Nt
                        const NttShape&, cudaStream_t st) {
   if (ls.count == 0) return cudaSuccess;
   if (log_n < kMinLogN || log_n > kMaxLogN) return cudaErrorInvalidValue;
-  return pick(log_n, ls.count, &Variant::ntt_upto).ntt(ls, mods, dir, st);
+  return pick(log_n, ls.count, &Variant::ntt_at).ntt(ls, mods, dir, st);
 }
 
 cudaError_t launch_polymul(const LimbSet& c, const ConstLimbSet& a, const ConstLimbSet& b,
@@ -209,7 +214,7 @@ cudaError_t launch_polymul(const LimbSet& c, const ConstLimbSet& a, const ConstL
                            const NttShape&, cudaStream_t st, uint64_t* const* scratch_ptrs) {
   if (c.count == 0) return cudaSuccess;
   if (log_n < kMinLogN || log_n > kMaxLogN) return cudaErrorInvalidValue;
-  const Variant* v = &pick(log_n, c.count, &Variant::polymul_upto);
+  const Variant* v = &pick(log_n, c.count, &Variant::polymul_at);
   if (v->polymul_scratch && scratch == nullptr && scratch_ptrs == nullptr) {
     // Without scratch, the first (selection order) variant that needs none.
     v = nullptr;

@@ -256,8 +256,8 @@ __global__ void __launch_bounds__(C::THREADS, C::THREADS <= 256 ? 3 : 1) k_ntt_w
   extern __shared__ __align__(16) uint64_t smem[];
   constexpr int K = C::K, NR = C::NR;
   const uint32_t log_n = K;
-  grid_dep_launch();
   grid_dep_wait();  // as in k_col_pass
+  grid_dep_launch();
   const uint32_t tid = threadIdx.x;
   const uint32_t limb0 = blockIdx.x << (C::T - K);
   const uint32_t my_limb = limb0 + C::sub(tid);
@@ -416,10 +416,10 @@ __global__ void __launch_bounds__(C::THREADS, min_blocks(INV ? 1024 : 768, C::TH
   constexpr int K = C::K, LB = C::LB, NR = C::NR;
   constexpr uint32_t log_n = K + LOGB;
   constexpr int TPL = LOGB - LB;  // log2(tiles per limb)
-  grid_dep_launch();
   // when launched as a dependent: the previous kernel's words, and limb or
   // modulus lists it may have written, are read only after this
   grid_dep_wait();
+  grid_dep_launch();
   const uint32_t tid = threadIdx.x;
   const uint32_t limb = dst.ordered(blockIdx.x >> TPL);
   const uint32_t col0 = (blockIdx.x & ((1u << TPL) - 1u)) << LB;
@@ -477,8 +477,8 @@ __global__ void __launch_bounds__(C::THREADS) k_row_pass(LimbSet ls, const DevMo
   constexpr int K = C::K, NR = C::NR;
   constexpr uint32_t log_n = K + K1;
   constexpr int TPL = log_n - C::T;
-  grid_dep_launch();
   grid_dep_wait();  // as in k_col_pass
+  grid_dep_launch();
   const uint32_t tid = threadIdx.x;
   const uint32_t limb = ls.ordered(blockIdx.x >> TPL);
   const uint32_t off = (blockIdx.x & ((1u << TPL) - 1u)) << C::T;
@@ -530,8 +530,8 @@ __global__ void __launch_bounds__(C::THREADS, min_blocks(INV ? 1024 : 896, C::TH
   constexpr int K = C::K, NR = C::NR;
   constexpr uint32_t log_n = K + K1;
   constexpr int TPL = log_n - C::T;
-  grid_dep_launch();
   grid_dep_wait();  // as in k_col_pass
+  grid_dep_launch();
   uint64_t* sa = smem;
   uint64_t* sb = smem + tile_smem_words(1u << C::T);
   const uint32_t tid = threadIdx.x;
@@ -679,8 +679,8 @@ __device__ __forceinline__ void polymul_whole_body(LimbSet c, ConstLimbSet a, Co
 template <class C>
 __global__ void __launch_bounds__(C::THREADS, C::THREADS <= 256 ? 2 : 1) k_polymul_whole(LimbSet c, ConstLimbSet a, ConstLimbSet b,
                                                               const DevMod* __restrict__ mods) {
-  grid_dep_launch();
   grid_dep_wait();  // as in k_col_pass
+  grid_dep_launch();
   polymul_whole_body<C>(c, a, b, mods, blockIdx.x);
 }
 
@@ -736,8 +736,8 @@ constexpr int two_operand_threads() { return C::LOGE == 4 ? 512 : 768; }
 template <class C, int LOGB, int SM_THREADS>
 __global__ void __launch_bounds__(C::THREADS, min_blocks(SM_THREADS, C::THREADS))
     k_col_pass2(ConstLimbSet a, ConstLimbSet b, LimbSet ca, LimbSet cb, const DevMod* __restrict__ mods) {
-  grid_dep_launch();
   grid_dep_wait();  // as in k_col_pass
+  grid_dep_launch();
   col_pass2_body<C, LOGB>(a, b, ca, cb, mods, blockIdx.x);
 }
 
@@ -789,8 +789,8 @@ __device__ __forceinline__ void polymul_rows_body(LimbSet ca, ConstLimbSet sbuf,
 template <class C, int K1>
 __global__ void __launch_bounds__(C::THREADS, min_blocks(two_operand_threads<C>(), C::THREADS))
     k_polymul_rows(LimbSet ca, ConstLimbSet sbuf, const DevMod* __restrict__ mods) {
-  grid_dep_launch();
   grid_dep_wait();  // as in k_col_pass
+  grid_dep_launch();
   // tiles in the reverse of the column pass's order: the first rows read the
   // words the column pass wrote last, still in L2, and the inverse column
   // pass (forward order) starts on the rows written last

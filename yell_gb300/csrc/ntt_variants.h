@@ -6,7 +6,7 @@
 // column stages k1 of the two-pass path (columns of 2^k1 words, rows of
 // 2^(log_n - k1) words), or one limb per thread-block cluster.  A degree for
 // which no variant was selected takes the one registered for the call's
-// number of limbs (polymul_upto, ntt_upto), else variant 0; the autotuner
+// number of limbs (polymul_at, ntt_at), else variant 0; the autotuner
 // times every variant of a degree on the current device and selects the
 // fastest, which then runs at every number of limbs.
 #pragma once
@@ -15,6 +15,10 @@
 #include "kernels.h"
 
 namespace yell_gb300 {
+
+struct LimbRange {
+  uint32_t least = 1, most = 0;  // none
+};
 
 struct Variant {
   char name[96] = {};
@@ -25,9 +29,9 @@ struct Variant {
   uint32_t ntt_launches = 0;
   uint32_t polymul_launches = 0;
   bool polymul_scratch = false;  // the polymul needs one operand's worth of scratch words
-  // Chosen without a selection for calls of at most this many limbs (0:
-  // never); among several, the one with the smallest such bound.
-  uint32_t polymul_upto = 0, ntt_upto = 0;
+  // Chosen without a selection for calls whose number of limbs lies in one of
+  // these ranges; among several variants, the one whose range ends first.
+  LimbRange polymul_at[2], ntt_at[2];
   // One of the variants for few limbs: never the stand-in for a polymul
   // called without scratch.
   bool few_limbs = false;
@@ -35,10 +39,14 @@ struct Variant {
 
 constexpr uint32_t kAnyLimbs = 0xFFFFFFFFu;
 
-// A variant for few limbs, with its bounds.
-inline Variant upto(Variant v, uint32_t polymul_limbs, uint32_t ntt_limbs) {
-  v.polymul_upto = polymul_limbs;
-  v.ntt_upto = ntt_limbs;
+// A variant for few limbs: polymuls of up to polymul_limbs, NTTs of up to
+// ntt_limbs, and one further range of each.
+inline Variant upto(Variant v, uint32_t polymul_limbs, uint32_t ntt_limbs, LimbRange polymul_also = {},
+                    LimbRange ntt_also = {}) {
+  v.polymul_at[0] = {1, polymul_limbs};
+  v.polymul_at[1] = polymul_also;
+  v.ntt_at[0] = {1, ntt_limbs};
+  v.ntt_at[1] = ntt_also;
   v.few_limbs = true;
   return v;
 }

@@ -18,7 +18,7 @@ void add_whole_variants_large(std::vector<Variant>* by) {
   by[12].push_back(whole_variant<12, 13>());
   by[13].push_back(whole_variant<13, 13>());
   by[13].push_back(two_pass_variant<13, 6>());
-  by[13].back().polymul_upto = by[13].back().ntt_upto = kAnyLimbs;
+  by[13].back().polymul_at[0] = by[13].back().ntt_at[0] = {1, kAnyLimbs};
   by[13].push_back(two_pass_variant<13, 7>());
 }
 
