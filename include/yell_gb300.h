@@ -426,10 +426,13 @@ int yell_poly_to_bigint(uint64_t* out, const uint64_t* const* limbs, uint32_t L,
  * butterflies (same output words) with a different split of the work: limbs
  * per CTA for whole-limb degrees, column/row split k1 for 2^13 and up
  * (2^13 has both kinds).
- * yell_autotune times the fused polymul of every variant of log_n on
- * synthetic data of the given size on the current device and selects the
- * fastest; with YELL_GB300_TUNE_FILE set the choice is saved there and
- * reloaded when the library first uses the device. */
+ * Some variants are for few limbs (small tiles, thread-block clusters); calls
+ * of few limbs take them by their number of limbs.  yell_autotune times the
+ * fused polymul of every other variant of log_n on synthetic data of the
+ * given size on the current device and selects the fastest for the calls that
+ * take none of those; with YELL_GB300_TUNE_FILE set the choice is saved there
+ * and reloaded when the library first uses the device.  yell_set_variant
+ * selects a variant for every call of the degree. */
 int yell_variant_count(uint32_t log_n, uint32_t* count);
 int yell_variant_name(uint32_t log_n, uint32_t variant, char* buf, size_t len);
 int yell_set_variant(uint32_t log_n, uint32_t variant);

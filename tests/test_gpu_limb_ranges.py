@@ -23,3 +23,15 @@ def test_both_sides_of_the_ranges(cuda, orc, log_n):
     r = subprocess.run([sys.executable, "-c", SCRIPT % (log_n, COUNTS[log_n])], cwd=root, env=env,
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "few limbs ok" in r.stdout, r.stdout[-500:] + r.stderr[-1500:]
+
+
+TUNED = SCRIPT.replace("digests = {}", "y.autotune(log_n, 1, 2)\ndigests = {}")
+
+
+@pytest.mark.parametrize("log_n,counts", [(10, [2, 4098]), (13, [16, 1000]), (14, [11, 40, 512]), (16, [2, 8, 200])])
+def test_tuned_degree_keeps_the_variants_for_few_limbs(cuda, orc, log_n, counts):
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = {k: v for k, v in os.environ.items() if k != "YELL_GB300_TUNE_FILE"}
+    r = subprocess.run([sys.executable, "-c", TUNED % (log_n, counts)], cwd=root, env=env,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "few limbs ok" in r.stdout, r.stdout[-500:] + r.stderr[-1500:]

@@ -113,7 +113,9 @@ int num_sms() {
 
 std::vector<Variant> g_table[kMaxLogN + 1];
 std::once_flag g_table_once;
-// Selected variant + 1, or 0 when none was selected.
+// Selected variant + 1, with kTuned when the autotuner selected it, or 0 when
+// none was selected.
+constexpr uint32_t kTuned = 0x80;
 std::array<std::array<std::atomic<uint8_t>, kMaxLogN + 1>, 64> g_selected{};
 
 void build_table() {
@@ -137,16 +139,20 @@ int current_device() {
 }
 
 // The variant a call of `limbs` limbs runs: the selected one, else the one
-// registered for that many limbs, else the first.
+// registered for that many limbs, else the first.  A variant that the
+// autotuner selected takes the first one's place, behind those for few limbs:
+// it was timed at one size (2^14 tuned at 32 limbs picked 4 words per thread,
+// at which an NTT of 512 limbs took 99 us against 77).
 const Variant& pick(uint32_t log_n, uint32_t limbs, LimbRange (Variant::*ranges)[2]) {
   const std::vector<Variant>& vs = variants_of(log_n);
   const uint32_t sel = g_selected[current_device()][log_n].load(std::memory_order_relaxed);
-  if (sel != 0 && sel <= vs.size()) return vs[sel - 1];
-  const Variant* best = &vs[0];
+  const bool tuned = (sel & kTuned) != 0;
+  if (sel != 0 && !tuned) return vs[sel - 1];
+  const Variant* best = &vs[tuned ? (sel & ~kTuned) - 1 : 0];
   uint64_t most = ~0ull;
   for (const Variant& v : vs)
     for (const LimbRange& r : v.*ranges)
-      if (r.least <= limbs && limbs <= r.most && r.most < most) {
+      if ((!tuned || v.few_limbs) && r.least <= limbs && limbs <= r.most && r.most < most) {
         best = &v;
         most = r.most;
       }
@@ -162,11 +168,11 @@ const std::vector<Variant>& variants_of(uint32_t log_n) {
 
 uint32_t selected_variant(int device, uint32_t log_n) {
   const uint32_t sel = g_selected[device][log_n].load(std::memory_order_relaxed);
-  return sel != 0 ? sel - 1 : 0;
+  return sel != 0 ? (sel & ~kTuned) - 1 : 0;
 }
 
-void select_variant(int device, uint32_t log_n, uint32_t v) {
-  g_selected[device][log_n].store((uint8_t)(v + 1), std::memory_order_relaxed);
+void select_variant(int device, uint32_t log_n, uint32_t v, bool tuned) {
+  g_selected[device][log_n].store((uint8_t)((v + 1) | (tuned ? kTuned : 0)), std::memory_order_relaxed);
 }
 
 cudaError_t init_kernel_attributes() {

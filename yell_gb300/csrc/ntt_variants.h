@@ -7,8 +7,10 @@
 // 2^(log_n - k1) words), or one limb per thread-block cluster.  A degree for
 // which no variant was selected takes the one registered for the call's
 // number of limbs (polymul_at, ntt_at), else variant 0; the autotuner
-// times every variant of a degree on the current device and selects the
-// fastest, which then runs at every number of limbs.
+// times every variant of a degree but those for few limbs on the current
+// device and selects the fastest, which then runs at every number of limbs
+// that no variant for few limbs is registered for.  A variant selected by
+// hand runs at every number of limbs.
 #pragma once
 #include <vector>
 
@@ -68,6 +70,6 @@ void add_cluster_variants(std::vector<Variant>* by_degree);      // 2^10 .. 2^14
 const std::vector<Variant>& variants_of(uint32_t log_n);
 // (0 when none was).
 uint32_t selected_variant(int device, uint32_t log_n);
-void select_variant(int device, uint32_t log_n, uint32_t v);
+void select_variant(int device, uint32_t log_n, uint32_t v, bool tuned);
 
 }  // namespace yell_gb300

@@ -66,7 +66,7 @@ void load_tuning(int dev) {
     if (log_n < kMinLogN || log_n > kMaxLogN) continue;
     const std::vector<Variant>& vs = variants_of(log_n);
     for (uint32_t v = 0; v < vs.size(); ++v)
-      if (vname == vs[v].name) select_variant(dev, log_n, v);
+      if (vname == vs[v].name) select_variant(dev, log_n, v, !vs[v].few_limbs);
   }
 }
 
@@ -98,7 +98,7 @@ int yell_set_variant(uint32_t log_n, uint32_t variant) {
   if (variant >= variants_of(log_n).size()) return fail(kInvalidArgument, "no such variant");
   DeviceContext* ctx = DeviceContext::current(&st);
   if (!ctx) return st;
-  select_variant(ctx->device(), log_n, variant);
+  select_variant(ctx->device(), log_n, variant, false);
   return kOk;
 }
 
@@ -143,6 +143,7 @@ int yell_autotune(uint32_t log_n, uint32_t L, uint32_t pairs, uint32_t* best, do
   uint32_t best_v = 0;
   double best_t = 1e30;
   for (uint32_t v = 0; v < vs.size() && e == cudaSuccess; ++v) {
+    if (vs[v].few_limbs) continue;  // chosen by a call's number of limbs
     float t = 1e30f;
     for (int rep = 0; rep < 4 && e == cudaSuccess; ++rep) {
       e = cudaEventRecord(e0, s);
@@ -162,7 +163,7 @@ int yell_autotune(uint32_t log_n, uint32_t L, uint32_t pairs, uint32_t* best, do
   cudaEventDestroy(e1);
   cudaFree(buf);
   if (e != cudaSuccess) return fail_cuda(e, "autotune run");
-  select_variant(ctx->device(), log_n, best_v);
+  select_variant(ctx->device(), log_n, best_v, true);
   persist(ctx->device(), log_n, vs[best_v].name);
   if (best) *best = best_v;
   if (best_ms) *best_ms = best_t;
