@@ -49,8 +49,8 @@ struct PlainLaunches {
 // g_dependent_launches is cleared): the kernel's CTAs may start while that
 // kernel's last CTAs finish, and wait (grid_dep_wait, common.cuh) before
 // they touch global memory other than the library's tables.  Used for the
-// NTT and polymul, the element-wise ops, the samplers, the tensor-core CRT
-// lift and the staged 32-bit polymul.
+// NTT, polymul and element-wise kernels of both word sizes, the samplers and
+// the tensor-core CRT lift.
 template <typename... KArgs, typename... Args>
 void launch_dependent(void (*kernel)(KArgs...), dim3 grid, uint32_t threads, size_t smem, cudaStream_t st,
                       Args... args) {

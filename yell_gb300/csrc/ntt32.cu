@@ -275,6 +275,8 @@ template <class C, int DIR>
 __global__ void __launch_bounds__(C::THREADS, 1024 / C::THREADS) k32_ntt(uint32_t* data, Limbs32 ls, const DevMod32* __restrict__ mods) {
   extern __shared__ __align__(16) uint32_t smem32[];
   constexpr int NR = C::NR;
+  grid_dep_wait();  // the stream's previous kernel may produce or read data
+  grid_dep_launch();
   const uint32_t tid = threadIdx.x;
   const uint32_t limb0 = blockIdx.x << (C::T - C::K);
   const uint32_t my_limb = limb0 + C::sub(tid);
@@ -298,6 +300,8 @@ __global__ void __launch_bounds__(C::THREADS, 1024 / C::THREADS) k32_polymul(uin
   constexpr int NR = C::NR, E = 1 << C::LOGE;
   using RB = Round<C, NR - 1>;
   static_assert(RB::R == C::LOGE && RB::BETA == 0 && RB::EB == 0, "bottom round must own contiguous words");
+  grid_dep_wait();  // the stream's previous kernel may produce a or b, or read c
+  grid_dep_launch();
   const uint32_t tid = threadIdx.x;
   const uint32_t limb0 = blockIdx.x << (C::T - C::K);
   const uint32_t my_limb = limb0 + C::sub(tid);
@@ -590,6 +594,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Staged32::THREADS, 1
 template <int OP>
 __global__ void k32_elementwise(uint32_t* dst, const uint32_t* a, const uint32_t* b, size_t total, uint32_t log_n,
                                 Limbs32 ls, const DevMod32* __restrict__ mods) {
+  grid_dep_launch();
+  grid_dep_wait();  // as above
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
     const uint32_t cm = ls.cm((uint32_t)(k >> log_n));
     const uint32_t p = __ldg(&mods[cm].p);
@@ -622,17 +628,20 @@ cudaError_t set_attrs32() {
   return e;
 }
 
+// As programmatic dependents, like the 64-bit kernels (GB300, polymul, us:
+// 1 limb of 2^9 8.2 -> 5.3, 1024 of 2^9 10.3 -> 7.5, 2000 of 2^12 75.8 -> 73.8;
+// forward NTT of 1024 limbs of 2^9 6.2 -> 4.0).
 template <int LOGN>
 cudaError_t launch32(int kind, uint32_t* c, const uint32_t* a, const uint32_t* b, const Limbs32& ls,
                      const DevMod32* mods, cudaStream_t st) {
   using CF = Cfg32<LOGN>;
   using C = typename CF::C;
   const uint32_t blocks = (ls.count + (1u << (C::T - LOGN)) - 1) >> (C::T - LOGN);
-  if (kind == 0) k32_ntt<C, 0><<<blocks, C::THREADS, CF::kSmem, st>>>(c, ls, mods);
-  else if (kind == 1) k32_ntt<C, 1><<<blocks, C::THREADS, CF::kSmem, st>>>(c, ls, mods);
+  if (kind == 0) launch_dependent(k32_ntt<C, 0>, blocks, C::THREADS, CF::kSmem, st, c, ls, mods);
+  else if (kind == 1) launch_dependent(k32_ntt<C, 1>, blocks, C::THREADS, CF::kSmem, st, c, ls, mods);
   if constexpr (LOGN < kLogMaxOneCta32) {  // at 2^13 clusters take every inverse and polymul
-    if (kind == 2) k32_ntt<C, 2><<<blocks, C::THREADS, CF::kSmem, st>>>(c, ls, mods);
-    else if (kind == 3) k32_polymul<C><<<blocks, C::THREADS, CF::kSmem, st>>>(c, a, b, ls, mods + kMaxModuli32);
+    if (kind == 2) launch_dependent(k32_ntt<C, 2>, blocks, C::THREADS, CF::kSmem, st, c, ls, mods);
+    else if (kind == 3) launch_dependent(k32_polymul<C>, blocks, C::THREADS, CF::kSmem, st, c, a, b, ls, mods + kMaxModuli32);
   }
   return cudaGetLastError();
 }
@@ -961,11 +970,11 @@ int yell32_dev_elementwise(int op, uint32_t* d_dst, const uint32_t* d_a, const u
   const int grid = (int)std::min<size_t>((total + 255) / 256, 152 * 16);
   LaunchScope ps("elementwise32", s);
   switch (op) {
-    case YELL_OP_MULMOD: k32_elementwise<YELL_OP_MULMOD><<<grid, 256, 0, s>>>(d_dst, d_a, d_b, total, log_n, ls, mods); break;
-    case YELL_OP_ADDMOD: k32_elementwise<YELL_OP_ADDMOD><<<grid, 256, 0, s>>>(d_dst, d_a, d_b, total, log_n, ls, mods); break;
-    case YELL_OP_SUBMOD: k32_elementwise<YELL_OP_SUBMOD><<<grid, 256, 0, s>>>(d_dst, d_a, d_b, total, log_n, ls, mods); break;
-    case YELL_OP_MULADD: k32_elementwise<YELL_OP_MULADD><<<grid, 256, 0, s>>>(d_dst, d_a, d_b, total, log_n, ls, mods); break;
-    default: k32_elementwise<YELL_OP_NEGATE><<<grid, 256, 0, s>>>(d_dst, d_a, d_b, total, log_n, ls, mods); break;
+    case YELL_OP_MULMOD: launch_dependent(k32_elementwise<YELL_OP_MULMOD>, grid, 256, 0, s, d_dst, d_a, d_b, total, log_n, ls, mods); break;
+    case YELL_OP_ADDMOD: launch_dependent(k32_elementwise<YELL_OP_ADDMOD>, grid, 256, 0, s, d_dst, d_a, d_b, total, log_n, ls, mods); break;
+    case YELL_OP_SUBMOD: launch_dependent(k32_elementwise<YELL_OP_SUBMOD>, grid, 256, 0, s, d_dst, d_a, d_b, total, log_n, ls, mods); break;
+    case YELL_OP_MULADD: launch_dependent(k32_elementwise<YELL_OP_MULADD>, grid, 256, 0, s, d_dst, d_a, d_b, total, log_n, ls, mods); break;
+    default: launch_dependent(k32_elementwise<YELL_OP_NEGATE>, grid, 256, 0, s, d_dst, d_a, d_b, total, log_n, ls, mods); break;
   }
   g_kernel_launches += 1;
   const cudaError_t e = cudaGetLastError();

@@ -2,12 +2,12 @@
 // thread, for calls whose limbs do not fill the chip with tiles of 2^12: more
 // CTAs, and a shorter chain per thread.  Past the bounds the exchanges that
 // the narrower rounds add cost more than the idle SMs.  GB300, polymul us
-// (tiles of 2^12 -> here): 18 limbs of 2^14 46.3 -> 14.9, 64 36.6; 8 of 2^15
-// 42.3 -> 15.5; 4 of 2^16 45.2 -> 16.3, 8 50.2 -> 27.1; 1 of 2^17 40.0 -> 12.4, 4
-// 53.5 -> 28.6; 2 of 2^18 55.9 -> 39.5; 1 of 2^20 62.7 -> 54.3; and at the upper
-// bounds 1024 limbs of 2^13 221 against 221, 256 of 2^14 122 against 122, 128
-// of 2^15 130 against 128, 256 of 2^16 515 against 511, 64 of 2^18 598 against
-// 577.
+// (tiles of 2^12 -> here): 16 limbs of 2^14 38.6 -> 14.3, 64 46.3 -> 36.6; 8 of
+// 2^15 40.4 -> 14.9; 4 of 2^16 42.8 -> 15.7, 8 50.2 -> 27.1; 1 of 2^17 38.2 ->
+// 11.8, 4 53.5 -> 28.6; 2 of 2^18 55.9 -> 39.5; 1 of 2^20 62.7 -> 54.3; and at
+// the upper bounds 1024 limbs of 2^13 221 against 221, 256 of 2^14 122 against
+// 122, 128 of 2^15 130 against 128, 256 of 2^16 515 against 511, 64 of 2^18 598
+// against 577.
 // Between 4 and 8 words per thread the number of CTAs decides, 2^(log_n - 10)
 // per limb with 256 or 128 threads.  Up to one per SM the shorter chain wins
 // (2 limbs of 2^16 12.2 us against 13.6); at two and three per SM CTAs of 4
