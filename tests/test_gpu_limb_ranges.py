@@ -12,8 +12,8 @@ from test_gpu_few_limbs import SCRIPT
 pytestmark = pytest.mark.gpu
 
 COUNTS = {10: [80, 81, 160, 161, 1024, 1025], 12: [48, 49],
-          13: [15, 16, 19, 20, 33, 34, 39, 40, 48, 49, 52, 53, 56], 14: [11, 12, 22, 23, 28, 29, 36, 37],
-          15: [4, 5, 11, 12, 14, 15], 16: [2, 3, 7, 10, 11], 17: [2, 3, 5]}
+          13: [15, 16, 19, 20, 33, 34, 39, 40, 48, 49, 52, 53, 56], 14: [11, 12, 28, 29, 128, 129, 192, 193],
+          15: [4, 5, 14, 15, 96, 97], 16: [2, 3, 7, 10, 11, 64, 65], 17: [2, 3, 5, 64, 65]}
 
 
 @pytest.mark.parametrize("log_n", sorted(COUNTS))
