@@ -290,7 +290,7 @@ __device__ __forceinline__ uint32_t sub_borrow(uint64_t a, uint64_t b, uint32_t 
 constexpr int kDigitTile = 8;  // 8: 72 registers, 0.77 ms at L = 32; 16: 114 registers, 0.87 ms
 
 template <int T>
-__global__ void __launch_bounds__(T) k_crt_lift(uint64_t* __restrict__ out, const uint64_t* __restrict__ in,
+__global__ void __launch_bounds__(T) k_crt_lift(uint64_t* out, const uint64_t* in,
                                                 uint32_t count, uint32_t L, uint32_t log_n,
                                                 const CrtConst* __restrict__ mods, const uint64_t* __restrict__ cof,
                                                 const uint64_t* __restrict__ qw, uint32_t W) {
@@ -298,6 +298,8 @@ __global__ void __launch_bounds__(T) k_crt_lift(uint64_t* __restrict__ out, cons
   uint64_t* ys = smem_crt;                                          // [L][T]
   uint32_t* cs = reinterpret_cast<uint32_t*>(smem_crt + (size_t)L * T);  // [L][kDigitTile + 1]
   constexpr int CT = kDigitTile + 1;
+  grid_dep_wait();  // the caller's words are read and written below
+  grid_dep_launch();
   const uint64_t coeffs = (uint64_t)count << log_n;
   const uint64_t g = (uint64_t)blockIdx.x * T + threadIdx.x;
   const bool live = g < coeffs;
@@ -439,8 +441,8 @@ int crt_lift(uint64_t* d_out, const uint64_t* d_in, uint32_t count, uint32_t L, 
   if (s != kOk) return s;
   // From 4 moduli up the tensor-core kernel is the faster one at every number
   // of coefficients (GB300, us, digit kernel -> tensor cores: 2^20
-  // coefficients, L = 3: 35 -> 41, 4: 53 -> 42, 8: 117 -> 48, 16: 286 -> 80,
-  // 32: 762 -> 143; 2^13, L = 3: 6.1 -> 4.1, 32: 35 -> 6); its digits are exact
+  // coefficients, L = 3: 33 -> 41, 4: 53 -> 42, 8: 117 -> 48, 16: 286 -> 80,
+  // 32: 762 -> 143; 2^13, L = 3: 3.7 -> 4.1, 32: 35 -> 6); its digits are exact
   // up to kMaxL moduli.
   if (t->image) {
     const cudaError_t me = launch_crt_mma(d_out, d_in, (uint64_t)count << log_n, L, log_n, t, st, device);
@@ -469,10 +471,17 @@ int crt_lift(uint64_t* d_out, const uint64_t* d_in, uint32_t count, uint32_t L, 
   const uint32_t blocks = (uint32_t)((coeffs + threads - 1) / threads);
   {
     LaunchScope ps("crt_lift", st);
+    // A dependent for few moduli (GB300, 2 moduli, 2^15 coefficients 6.1 -> 3.8
+    // us, 2^20 28.5 -> 25.6).  With more than 32 its long CTAs, placed while the
+    // previous kernel's hold their SMs, pack unevenly: 2^16 coefficients, 33
+    // moduli, 76 us plainly and 102 as a dependent.
+    const bool dependent = g_dependent_launches;
+    g_dependent_launches = dependent && L < kMmaMinModuli;
     if (threads == 64)
-      k_crt_lift<64><<<blocks, 64, smem, st>>>(d_out, d_in, count, L, log_n, t->mods, t->cofactors, t->q, t->W);
+      launch_dependent(k_crt_lift<64>, blocks, 64, smem, st, d_out, d_in, count, L, log_n, t->mods, t->cofactors, t->q, t->W);
     else
-      k_crt_lift<32><<<blocks, 32, smem, st>>>(d_out, d_in, count, L, log_n, t->mods, t->cofactors, t->q, t->W);
+      launch_dependent(k_crt_lift<32>, blocks, 32, smem, st, d_out, d_in, count, L, log_n, t->mods, t->cofactors, t->q, t->W);
+    g_dependent_launches = dependent;
     g_kernel_launches += 1;
   }
   e = cudaGetLastError();

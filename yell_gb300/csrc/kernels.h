@@ -50,7 +50,7 @@ struct PlainLaunches {
 // kernel's last CTAs finish, and wait (grid_dep_wait, common.cuh) before
 // they touch global memory other than the library's tables.  Used for the
 // NTT, polymul and element-wise kernels of both word sizes, the samplers and
-// the tensor-core CRT lift.
+// the CRT lift of up to 32 moduli.
 template <typename... KArgs, typename... Args>
 void launch_dependent(void (*kernel)(KArgs...), dim3 grid, uint32_t threads, size_t smem, cudaStream_t st,
                       Args... args) {
