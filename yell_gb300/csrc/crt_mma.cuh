@@ -191,7 +191,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
   const uint32_t tmem_cols = N <= 16 ? 32u : (N <= 32 ? 64u : (N <= 64 ? 128u : (N <= 128 ? 256u : 512u)));
   const uint32_t tiles = (uint32_t)((coeffs + kRows - 1) / kRows);
-  grid_dep_launch();
 
   // once per CTA: constant matrix, moduli, barriers, TMEM
   {
@@ -219,6 +218,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     mbar_init(&bars->done, 1);
     bars->gave_up = 0;
   }
+  // The caller's words are read and written below.  TMEM is taken only now:
+  // a CTA that holds columns while it waits could keep them from a CTA of the
+  // kernel that it waits for.  For the same reason the next kernel may start
+  // only once this CTA has its columns.
+  grid_dep_wait();
   if (warp == kEpilogueWarps + kProducerWarps) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      (uint32_t)__cvta_generic_to_shared(&bars->tmem)),
@@ -230,8 +234,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   fence_before();
   __syncthreads();
   fence_after();
+  grid_dep_launch();
   const uint32_t tmem = *(volatile uint32_t*)&bars->tmem;
-  grid_dep_wait();  // the caller's words are read and written below
 
   if (warp >= kEpilogueWarps && warp < kEpilogueWarps + kProducerWarps) {
     // ---- producers: thread (row, part) takes moduli 8 c + kMine part .. of each chunk c
