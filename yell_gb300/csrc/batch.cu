@@ -235,8 +235,8 @@ int BatchExecutor::reserve_queue_ctl(size_t words) {
   }
   const size_t want = std::max<size_t>(words, 4096) * 2;
   cudaError_t e = lib_malloc(&d_queue_ctl_, want * sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMemset(d_queue_ctl_, 0, want * sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMemcpy(d_queue_ctl_, &status, 4, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = upload_zeros(d_queue_ctl_, want * sizeof(uint32_t));
+  if (e == cudaSuccess) e = upload(d_queue_ctl_, &status, 4);
   if (e != cudaSuccess) return fail_cuda(e, "cudaMalloc(queue control)");
   queue_ctl_words_ = want;
   return kOk;
@@ -390,7 +390,7 @@ int BatchExecutor::queue_status(cudaStream_t s, uint32_t* status) {
   if (!d_queue_ctl_) return kOk;
   cudaError_t e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = cudaMemcpy(status, d_queue_ctl_, 4, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemset(d_queue_ctl_, 0, 4);
+  if (e == cudaSuccess) e = upload_zeros(d_queue_ctl_, 4);
   return e == cudaSuccess ? kOk : fail_cuda(e, "queue status");
 }
 

@@ -204,9 +204,9 @@ int build_crt_tables(uint32_t cm0, uint32_t L, CrtTables* t) {
   cudaError_t e = lib_malloc(&t->mods, L * sizeof(CrtConst));
   if (e == cudaSuccess) e = lib_malloc(&t->cofactors, cof.size() * 8);
   if (e == cudaSuccess) e = lib_malloc(&t->q, (size_t)W * 8);
-  if (e == cudaSuccess) e = cudaMemcpy(t->mods, mods.data(), L * sizeof(CrtConst), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(t->cofactors, cof.data(), cof.size() * 8, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(t->q, Q.data(), (size_t)W * 8, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = upload(t->mods, mods.data(), L * sizeof(CrtConst));
+  if (e == cudaSuccess) e = upload(t->cofactors, cof.data(), cof.size() * 8);
+  if (e == cudaSuccess) e = upload(t->q, Q.data(), (size_t)W * 8);
   if (e == cudaSuccess && L >= kMmaMinModuli && L <= crt_mma::kMaxL) {
     std::vector<crt_mma::Mod> mm(L);
     for (uint32_t j = 0; j < L; ++j)
@@ -215,8 +215,8 @@ int build_crt_tables(uint32_t cm0, uint32_t L, CrtTables* t) {
     e = lib_malloc(&t->mma_mods, L * sizeof(crt_mma::Mod));
     if (e == cudaSuccess) e = lib_malloc(&t->image, img.size());
     if (e == cudaSuccess)
-      e = cudaMemcpy(t->mma_mods, mm.data(), L * sizeof(crt_mma::Mod), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(t->image, img.data(), img.size(), cudaMemcpyHostToDevice);
+      e = upload(t->mma_mods, mm.data(), L * sizeof(crt_mma::Mod));
+    if (e == cudaSuccess) e = upload(t->image, img.data(), img.size());
   }
   if (e != cudaSuccess) {
     cudaFree(t->mods);
@@ -533,8 +533,9 @@ int yell_crt_wait_status(uint32_t* status) {
   e = cudaMemcpyFromSymbol(&v, g_crt_wait_status, sizeof(v));
   if (e != cudaSuccess) return fail_cuda(e, "read wait status");
   if (v != 0) {
-    const uint32_t zero = 0;
-    e = cudaMemcpyToSymbol(g_crt_wait_status, &zero, sizeof(zero));
+    void* word = nullptr;
+    e = cudaGetSymbolAddress(&word, g_crt_wait_status);
+    if (e == cudaSuccess) e = upload_zeros(word, sizeof(v));
     if (e != cudaSuccess) return fail_cuda(e, "clear wait status");
   }
   *status = v;

@@ -102,6 +102,19 @@ cudaError_t lib_malloc_async(T** p, size_t bytes, cudaMemPool_t pool, cudaStream
   return e;
 }
 
+// Host words to device memory, and zeros, that later work of any stream reads:
+// on the device when the call returns.  A copy from pageable memory may return
+// once the words are staged and a memset before it ran, both on the default
+// stream, for which the library's own non-blocking streams do not wait.
+inline cudaError_t upload(void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
+}
+inline cudaError_t upload_zeros(void* dst, size_t bytes) {
+  const cudaError_t e = cudaMemset(dst, 0, bytes);
+  return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
+}
+
 // In-place NTT over every limb of `ls`.  mods: the DevMod array of this
 // degree, indexed by modulus index.
 cudaError_t launch_ntt(const LimbSet& ls, uint32_t log_n, const DevMod* mods, NttDir dir,

@@ -167,7 +167,7 @@ int ensure32(int device, uint32_t log_n, uint32_t cm0, uint32_t L, const DevMod3
       t.mods[log_n] = nullptr;
       return fail_cuda(e, "cudaMalloc(DevMod32 table)");
     }
-    e = cudaMemset(t.mods[log_n], 0, 2 * kMaxModuli32 * sizeof(DevMod32));
+    e = upload_zeros(t.mods[log_n], 2 * kMaxModuli32 * sizeof(DevMod32));
     if (e != cudaSuccess) return fail_cuda(e, "cudaMemset(DevMod32 table)");
   }
   const uint32_t n = 1u << log_n;
@@ -185,7 +185,7 @@ int ensure32(int device, uint32_t log_n, uint32_t cm0, uint32_t L, const DevMod3
     uint32_t* d = nullptr;
     e = lib_malloc(&d, packed.size() * sizeof(uint32_t));
     if (e != cudaSuccess) return fail_cuda(e, "cudaMalloc(twiddles32)");
-    e = cudaMemcpy(d, packed.data(), packed.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    e = upload(d, packed.data(), packed.size() * sizeof(uint32_t));
     if (e != cudaSuccess) return fail_cuda(e, "upload twiddles32");
     DevMod32 m;
     m.fwd = reinterpret_cast<const uint2*>(d);
@@ -196,7 +196,7 @@ int ensure32(int device, uint32_t log_n, uint32_t cm0, uint32_t L, const DevMod3
     m.inv_n_s = sc[1];
     m.inv_n_iphi = sc[2];
     m.inv_n_iphi_s = sc[3];
-    e = cudaMemcpy(t.mods[log_n] + cm, &m, sizeof m, cudaMemcpyHostToDevice);
+    e = upload(t.mods[log_n] + cm, &m, sizeof m);
     if (e != cudaSuccess) return fail_cuda(e, "upload DevMod32");
     DevMod32 pm = m;
     uint32_t inv = m.p;  // p * p = 1 mod 8; Newton's iteration doubles the correct low bits
@@ -207,7 +207,7 @@ int ensure32(int device, uint32_t log_n, uint32_t cm0, uint32_t L, const DevMod3
     pm.inv_n_s = shoupify32(pm.inv_n, m.p);
     pm.inv_n_iphi = (uint32_t)(m.inv_n_iphi * r32 % m.p);
     pm.inv_n_iphi_s = shoupify32(pm.inv_n_iphi, m.p);
-    e = cudaMemcpy(t.mods[log_n] + kMaxModuli32 + cm, &pm, sizeof pm, cudaMemcpyHostToDevice);
+    e = upload(t.mods[log_n] + kMaxModuli32 + cm, &pm, sizeof pm);
     if (e != cudaSuccess) return fail_cuda(e, "upload DevMod32");
     built[cm] = 1;
   }
@@ -945,8 +945,9 @@ int yell32_wait_status(uint32_t* status) {
   e = cudaMemcpyFromSymbol(&v, g_k32_wait_status, sizeof(v));
   if (e != cudaSuccess) return fail_cuda(e, "read wait status");
   if (v != 0) {
-    const uint32_t zero = 0;
-    e = cudaMemcpyToSymbol(g_k32_wait_status, &zero, sizeof(zero));
+    void* word = nullptr;
+    e = cudaGetSymbolAddress(&word, g_k32_wait_status);
+    if (e == cudaSuccess) e = upload_zeros(word, sizeof(v));
     if (e != cudaSuccess) return fail_cuda(e, "clear wait status");
   }
   *status = v;

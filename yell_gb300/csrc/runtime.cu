@@ -309,7 +309,7 @@ int DeviceContext::ensure_tables_list(uint32_t log_n, const uint32_t* cms, uint3
       d_mods_[log_n] = nullptr;
       return fail_cuda(e, "cudaMalloc(DevMod table)");
     }
-    e = cudaMemset(d_mods_[log_n], 0, 2 * kMaxModuli * sizeof(DevMod));
+    e = upload_zeros(d_mods_[log_n], 2 * kMaxModuli * sizeof(DevMod));
     if (e != cudaSuccess) return fail_cuda(e, "cudaMemset(DevMod table)");
   }
   const uint32_t nwords = 1u << log_n;
@@ -346,7 +346,7 @@ int DeviceContext::ensure_tables_list(uint32_t log_n, const uint32_t* cms, uint3
     e = lib_malloc(&dtab, packed.size() * sizeof(uint64_t));
     if (e != cudaSuccess) return fail_cuda(e, "cudaMalloc(twiddle table)");
     table_allocs_.push_back(dtab);
-    e = cudaMemcpy(dtab, packed.data(), packed.size() * sizeof(uint64_t), cudaMemcpyHostToDevice);
+    e = upload(dtab, packed.data(), packed.size() * sizeof(uint64_t));
     if (e != cudaSuccess) return fail_cuda(e, "cudaMemcpy(twiddle table)");
     DevMod m;
     m.fwd = reinterpret_cast<const ulonglong2*>(dtab);
@@ -357,7 +357,7 @@ int DeviceContext::ensure_tables_list(uint32_t log_n, const uint32_t* cms, uint3
     m.inv_n_s = sc[4 * i + 1];
     m.inv_n_iphi = sc[4 * i + 2];
     m.inv_n_iphi_s = sc[4 * i + 3];
-    e = cudaMemcpy(d_mods_[log_n] + cm, &m, sizeof(DevMod), cudaMemcpyHostToDevice);
+    e = upload(d_mods_[log_n] + cm, &m, sizeof(DevMod));
     if (e != cudaSuccess) return fail_cuda(e, "cudaMemcpy(DevMod)");
     // the fused polymul's copy: Montgomery constant, inverse scaling times 2^64
     DevMod pm = m;
@@ -367,7 +367,7 @@ int DeviceContext::ensure_tables_list(uint32_t log_n, const uint32_t* cms, uint3
     pm.inv_n_s = shoupify(pm.inv_n, m.p);
     pm.inv_n_iphi = mulmod_exact(m.inv_n_iphi, r64, m.p);
     pm.inv_n_iphi_s = shoupify(pm.inv_n_iphi, m.p);
-    e = cudaMemcpy(d_mods_[log_n] + kPolymulConsts + cm, &pm, sizeof(DevMod), cudaMemcpyHostToDevice);
+    e = upload(d_mods_[log_n] + kPolymulConsts + cm, &pm, sizeof(DevMod));
     if (e != cudaSuccess) return fail_cuda(e, "cudaMemcpy(DevMod)");
     built[cm] = 1;
   }

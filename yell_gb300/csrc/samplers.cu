@@ -446,7 +446,7 @@ int gaussian_table(int device, double sigma, uint32_t tail, const uint64_t** out
     uint64_t* d = nullptr;
     cudaError_t e = lib_malloc(&d, cdt.size() * sizeof(uint64_t));
     if (e != cudaSuccess) return fail_cuda(e, "cudaMalloc(gaussian table)");
-    e = cudaMemcpy(d, cdt.data(), cdt.size() * sizeof(uint64_t), cudaMemcpyHostToDevice);
+    e = upload(d, cdt.data(), cdt.size() * sizeof(uint64_t));
     if (e != cudaSuccess) {
       cudaFree(d);
       return fail_cuda(e, "upload gaussian table");
