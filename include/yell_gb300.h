@@ -411,14 +411,22 @@ int yell_crt_words(uint32_t L, uint32_t cm0, uint32_t* words);
 /* d_in: count polys (count, L, N); d_out: count * N * W words. */
 int yell_dev_crt_lift(uint64_t* d_out, const uint64_t* d_in, uint32_t count, uint32_t L, uint32_t log_n,
                       uint32_t cm0, void* stream);
-/* With 4 to 32 moduli the lift's CTAs wait on the device for one another's
- * warps, each wait for at most 1 s; one that runs out records
- * YELL_ERR_TIMEOUT and the kernel still finishes (its output is then
- * undefined).  This call waits for all work queued on the current device,
- * stores the recorded status (YELL_OK or YELL_ERR_TIMEOUT) in *status and
- * clears it. */
+/* With 4 to 32 moduli the warps of the lift's CTAs wait on the device for one
+ * another, each wait for at most 1 s (time in which the process does not run
+ * on the device does not count); one that runs out records YELL_ERR_TIMEOUT
+ * and the kernel still finishes (its output is then undefined).  This call
+ * waits for all work queued on the current device, stores the status recorded
+ * by lifts of device arrays since the last such call, from any thread (YELL_OK
+ * or YELL_ERR_TIMEOUT), in *status and clears it. */
 int yell_crt_wait_status(uint32_t* status);
-/* Host drop-in for poly2mpz over moduli 0 .. L-1: limbs[j] -> out (N * W words). */
+/* Check of that bounded wait: a one-CTA kernel waits twice for what nobody
+ * signals; the first wait runs out after timeout_ns (<= 10 s), the second
+ * returns at once, and *status receives YELL_ERR_TIMEOUT (read and cleared as
+ * by yell_crt_wait_status).  Synchronous. */
+int yell_crt_wait_check(uint64_t timeout_ns, uint32_t* status);
+/* Host drop-in for poly2mpz over moduli 0 .. L-1: limbs[j] -> out (N * W
+ * words).  Returns YELL_ERR_TIMEOUT, with out undefined, when a wait of its
+ * own lift ran out. */
 int yell_poly_to_bigint(uint64_t* out, const uint64_t* const* limbs, uint32_t L, uint32_t log_n);
 
 /* ---- launch variants and the autotuner (no counterpart in the reference) --

@@ -109,6 +109,7 @@ SIGNATURES = {
     "yell32_dev_polymul": (_int, [_vp, _vp, _vp, _u32, _u32, _u32, _u32, _vp]),
     "yell32_wait_status": (_int, [_vp]),
     "yell_crt_wait_status": (_int, [_vp]),
+    "yell_crt_wait_check": (_int, [_u64, _vp]),
     "yell32_wait_check": (_int, [_u64, _vp]),
     "yell32_dev_elementwise": (_int, [_int, _vp, _vp, _vp, _u32, _u32, _u32, _u32, _vp]),
     "yell32_poly_forward": (_int, [_vp, _u32, _u32]),

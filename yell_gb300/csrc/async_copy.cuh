@@ -52,23 +52,49 @@ __device__ __forceinline__ bool mbar_test(uint64_t* mbar, uint32_t parity) {
   return done != 0;
 }
 
+// The same, suspended for no longer than the device chooses.
+__device__ __forceinline__ bool mbar_poll(uint64_t* mbar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"((uint32_t)__cvta_generic_to_shared(mbar)), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
+// Waits for phase `parity` of the mbarrier until it has polled for `limit`
+// units of 1024 ns or 2^24 times; a time in which the context does not run
+// counts for 2 ms at most (64 polls of a barrier that stands still take 0.25 ms
+// on GB300).  When a limit runs out it records `timeout_code` in *status (if
+// still 0) and returns false.  In 32-bit arithmetic: a caller's registers are
+// live around it.
+__device__ __forceinline__ bool mbar_wait_running(uint64_t* mbar, uint32_t parity, uint32_t* status,
+                                                  uint32_t timeout_code, uint32_t limit) {
+  uint32_t last = (uint32_t)globaltimer_ns(), spent = 0;
+  for (uint32_t i = 1; i <= (1u << 24); ++i) {
+    if (mbar_poll(mbar, parity)) return true;
+    if ((i & 63u) == 0) {
+      const uint32_t now = (uint32_t)globaltimer_ns();
+      spent += min(now - last, 2000000u) >> 10;
+      last = now;
+      if (spent > limit) break;
+    }
+  }
+  atomicCAS(status, 0u, timeout_code);
+  return false;
+}
+
 // Waits for phase `parity` of the mbarrier for at most timeout_ns of the
 // global timer (1 s unless given) or 2^24 polls.  When either limit runs out
 // it records `timeout_code` in *status (if still 0) and returns false.
 __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint32_t* status,
                                           uint32_t timeout_code, uint64_t timeout_ns = 1000000000ull) {
-  const uint32_t a = (uint32_t)__cvta_generic_to_shared(mbar);
   const uint64_t t0 = globaltimer_ns();
   for (uint32_t i = 0; i < (1u << 24); ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
+    if (mbar_poll(mbar, parity)) return true;
     if ((i & 255u) == 255u && globaltimer_ns() - t0 > timeout_ns) break;
   }
   if (status) atomicCAS(status, 0u, timeout_code);

@@ -395,18 +395,19 @@ size_t crt_smem(uint32_t L, int threads) {
   return (size_t)L * threads * sizeof(uint64_t) + (size_t)L * (kDigitTile + 1) * sizeof(uint32_t);
 }
 
-// First status of a bounded wait of the tensor-core kernel.
+// First status of a bounded wait of the tensor-core kernel, for the lifts of
+// device arrays; a host call has a word of its own.
 __device__ uint32_t g_crt_wait_status;
 
 cudaError_t launch_crt_mma(uint64_t* d_out, const uint64_t* d_in, uint64_t coeffs, uint32_t L, uint32_t log_n,
-                           const CrtTables* t, cudaStream_t st, int device) {
+                           const CrtTables* t, cudaStream_t st, int device, uint32_t* own_status) {
   using namespace crt_mma;
   static constexpr decltype(&k_crt_mma<1>) kKernels[] = {k_crt_mma<1>, k_crt_mma<2>, k_crt_mma<3>, k_crt_mma<4>};
   static_assert(sizeof(kKernels) / sizeof(kKernels[0]) == chunks(kMaxL), "a kernel per number of chunks");
   static std::mutex mu;
   static std::map<int, std::pair<uint32_t, uint32_t*>> devices;  // SMs and the status word's address
   uint32_t sms = 0;
-  uint32_t* status = nullptr;
+  uint32_t* status = own_status;
   {
     std::lock_guard<std::mutex> g(mu);
     auto it = devices.find(device);
@@ -423,7 +424,7 @@ cudaError_t launch_crt_mma(uint64_t* d_out, const uint64_t* d_in, uint64_t coeff
       it = devices.emplace(device, std::make_pair((uint32_t)n, static_cast<uint32_t*>(p))).first;
     }
     sms = it->second.first;
-    status = it->second.second;
+    if (!status) status = it->second.second;
   }
   const uint64_t tiles = (coeffs + kRows - 1) / kRows;
   const uint32_t grid = (uint32_t)(tiles < sms ? tiles : sms);
@@ -434,8 +435,25 @@ cudaError_t launch_crt_mma(uint64_t* d_out, const uint64_t* d_in, uint64_t coeff
   return cudaGetLastError();
 }
 
+// Reads a word that waits are recorded in, after the work queued on `st`, and
+// clears it.
+cudaError_t take_status(uint32_t* word, cudaStream_t st, uint32_t* status) {
+  uint32_t v = 0;
+  cudaError_t e = cudaMemcpyAsync(&v, word, sizeof(v), cudaMemcpyDeviceToHost, st);
+  const cudaError_t se = cudaStreamSynchronize(st);  // v is written until then
+  if (e == cudaSuccess) e = se;
+  if (e == cudaSuccess && v != 0) {
+    e = cudaMemsetAsync(word, 0, sizeof(v), st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  }
+  *status = v;
+  return e;
+}
+
+// own_status: the word of device memory that a wait of the tensor-core kernel
+// which runs out is recorded in, nullptr for the device's.
 int crt_lift(uint64_t* d_out, const uint64_t* d_in, uint32_t count, uint32_t L, uint32_t log_n, uint32_t cm0,
-             cudaStream_t st, int device) {
+             cudaStream_t st, int device, uint32_t* own_status) {
   const CrtTables* t = nullptr;
   int s = crt_tables(device, cm0, L, &t);
   if (s != kOk) return s;
@@ -445,7 +463,7 @@ int crt_lift(uint64_t* d_out, const uint64_t* d_in, uint32_t count, uint32_t L, 
   // 32: 762 -> 143; 2^13, L = 3: 3.7 -> 4.1, 32: 35 -> 6); its digits are exact
   // up to kMaxL moduli.
   if (t->image) {
-    const cudaError_t me = launch_crt_mma(d_out, d_in, (uint64_t)count << log_n, L, log_n, t, st, device);
+    const cudaError_t me = launch_crt_mma(d_out, d_in, (uint64_t)count << log_n, L, log_n, t, st, device, own_status);
     return me == cudaSuccess ? kOk : fail_cuda(me, "crt_lift");
   }
   // 64 threads per block while their y_j fit in 160 KB of shared memory, else 32
@@ -519,7 +537,7 @@ int yell_dev_crt_lift(uint64_t* d_out, const uint64_t* d_in, uint32_t count, uin
   DeviceContext* ctx = DeviceContext::current(&st);
   if (!ctx) return st;
   return crt_lift(d_out, d_in, count, L, log_n, cm0, stream ? static_cast<cudaStream_t>(stream) : ctx->stream(),
-                  ctx->device());
+                  ctx->device(), nullptr);
 }
 
 int yell_crt_wait_status(uint32_t* status) {
@@ -528,18 +546,26 @@ int yell_crt_wait_status(uint32_t* status) {
   DeviceContext* ctx = DeviceContext::current(&st);
   if (!ctx) return st;
   cudaError_t e = cudaDeviceSynchronize();
-  if (e != cudaSuccess) return fail_cuda(e, "synchronize");
-  uint32_t v = 0;
-  e = cudaMemcpyFromSymbol(&v, g_crt_wait_status, sizeof(v));
-  if (e != cudaSuccess) return fail_cuda(e, "read wait status");
-  if (v != 0) {
-    void* word = nullptr;
-    e = cudaGetSymbolAddress(&word, g_crt_wait_status);
-    if (e == cudaSuccess) e = upload_zeros(word, sizeof(v));
-    if (e != cudaSuccess) return fail_cuda(e, "clear wait status");
-  }
-  *status = v;
-  return kOk;
+  void* word = nullptr;
+  if (e == cudaSuccess) e = cudaGetSymbolAddress(&word, g_crt_wait_status);
+  if (e == cudaSuccess) e = take_status(static_cast<uint32_t*>(word), ctx->stream(), status);
+  return e == cudaSuccess ? kOk : fail_cuda(e, "read wait status");
+}
+
+int yell_crt_wait_check(uint64_t timeout_ns, uint32_t* status) {
+  if (!status) return fail(kInvalidArgument, "null output");
+  if (timeout_ns == 0 || timeout_ns > 10'000'000'000ull) return fail(kInvalidArgument, "timeout must be in (0, 10 s]");
+  int st = kOk;
+  DeviceContext* ctx = DeviceContext::current(&st);
+  if (!ctx) return st;
+  void* word = nullptr;
+  cudaError_t e = cudaGetSymbolAddress(&word, g_crt_wait_status);
+  if (e != cudaSuccess) return fail_cuda(e, "wait check");
+  crt_mma::k_crt_wait_check<<<1, 64, 0, ctx->stream()>>>((uint32_t)(timeout_ns >> 10) + 1, static_cast<uint32_t*>(word));
+  g_kernel_launches += 1;
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return fail_cuda(e, "wait check");
+  return yell_crt_wait_status(status);
 }
 
 int yell_poly_to_bigint(uint64_t* out, const uint64_t* const* limbs, uint32_t L, uint32_t log_n) {
@@ -553,20 +579,23 @@ int yell_poly_to_bigint(uint64_t* out, const uint64_t* const* limbs, uint32_t L,
   const size_t n = (size_t)1 << log_n;
   const uint32_t W = crt_words(0, L);
   std::lock_guard<std::mutex> g(ctx->staging.lock);
-  st = ctx->staging.reserve(n * L + n * W);
+  st = ctx->staging.reserve(n * L + n * W + 1);
   if (st != kOk) return st;
   cudaStream_t s = ctx->stream();
   uint64_t* d_in = ctx->staging.ptr;
   uint64_t* d_out = d_in + n * L;
-  cudaError_t e = cudaSuccess;
+  uint32_t* d_status = reinterpret_cast<uint32_t*>(d_out + n * W);
+  uint32_t status = kOk;
+  cudaError_t e = cudaMemsetAsync(d_status, 0, sizeof(status), s);
   for (uint32_t j = 0; j < L && e == cudaSuccess; ++j)
     e = cudaMemcpyAsync(d_in + j * n, limbs[j], n * 8, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return fail_cuda(e, "H2D limbs");
-  st = crt_lift(d_out, d_in, 1, L, log_n, 0, s, ctx->device());
+  st = crt_lift(d_out, d_in, 1, L, log_n, 0, s, ctx->device(), d_status);
   if (st != kOk) return st;
   e = cudaMemcpyAsync(out, d_out, n * W * 8, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  return e == cudaSuccess ? kOk : fail_cuda(e, "D2H / synchronize");
+  if (e == cudaSuccess) e = take_status(d_status, s, &status);
+  if (e != cudaSuccess) return fail_cuda(e, "D2H / synchronize");
+  return status == kOk ? kOk : fail((int)status, "CRT lift: a wait on the device ran out, the words are undefined");
 }
 
 }  // extern "C"

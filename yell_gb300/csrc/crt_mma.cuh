@@ -161,19 +161,43 @@ __device__ __forceinline__ uint4 digits_f16(int64_t y) {
 
 struct Bars {
   uint64_t full[kRing], empty[kRing], tail_full[kTails], tail_empty[kTails], acc_full[2], acc_empty[2], done;
-  uint32_t tmem, gave_up;
+  uint32_t tmem, gave_up, limit;  // limit: wait<0>
 };
 static_assert(sizeof(Bars) <= 256, "barrier block");
 
 // A bounded wait (1 s).  The first one to run out records YELL_ERR_TIMEOUT
 // and lets the CTA's other waits return at once: the CTA still reaches its
-// end, with its output undefined.
+// end, with its output undefined.  Only time in which the wait polls counts:
+// what it waits for is done by warps of the same CTA, which stand still with
+// it while a debugger or another process has the device.
+constexpr uint32_t kWaitLimit = 1000000000u >> 10;  // in units of 1024 ns
+// LIMIT 0: the limit is b->limit (read from shared memory it costs the lift of
+// 32 moduli a spill).
+template <uint32_t LIMIT>
 __device__ __noinline__ void wait_slow(Bars* b, uint64_t* mbar, uint32_t parity, uint32_t* status) {
-  if (*(volatile uint32_t*)&b->gave_up) return;
-  if (!mbar_wait(mbar, parity, status, (uint32_t)YELL_ERR_TIMEOUT)) *(volatile uint32_t*)&b->gave_up = 1;
+  if (*(volatile uint32_t*)&b->gave_up && mbar != &b->done) return;  // work in flight is waited for in any case
+  if (!mbar_wait_running(mbar, parity, status, (uint32_t)YELL_ERR_TIMEOUT, LIMIT ? LIMIT : b->limit))
+    *(volatile uint32_t*)&b->gave_up = 1;
 }
+template <uint32_t LIMIT = kWaitLimit>
 __device__ __forceinline__ void wait(Bars* b, uint64_t* mbar, uint32_t parity, uint32_t* status) {
-  if (!mbar_test(mbar, parity)) wait_slow(b, mbar, parity, status);
+  if (!mbar_test(mbar, parity)) wait_slow<LIMIT>(b, mbar, parity, status);
+}
+
+// Check of the bounded wait: one CTA waits twice on a barrier at which nobody
+// arrives.  The first wait runs out and records YELL_ERR_TIMEOUT, the second
+// returns at once.
+__global__ void k_crt_wait_check(uint32_t limit, uint32_t* status) {
+  __shared__ Bars bars;
+  if (threadIdx.x == 0) {
+    mbar_init(&bars.full[0], 1);
+    bars.gave_up = 0;
+    bars.limit = limit;
+  }
+  __syncthreads();
+  wait<0>(&bars, &bars.full[0], 0, status);
+  __syncthreads();
+  wait<0>(&bars, &bars.full[0], 0, status);
 }
 
 // image: image_bytes(L, N) bytes in operand layout; mods: L entries.
@@ -378,10 +402,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         ++tr;
       }
     }
-    if (leader) {
-      mma_commit(&bars->done);
-      bars->gave_up = 0;  // the work in flight is waited for in any case
-    }
+    if (leader) mma_commit(&bars->done);
     __syncwarp();
     wait(bars, &bars->done, 0, status);
     __syncwarp();
