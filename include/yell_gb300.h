@@ -440,11 +440,18 @@ int yell_poly_to_bigint(uint64_t* out, const uint64_t* const* limbs, uint32_t L,
  * given size on the current device and selects the fastest for the calls that
  * take none of those; with YELL_GB300_TUNE_FILE set the choice is saved there
  * and reloaded when the library first uses the device.  yell_set_variant
- * selects a variant for every call of the degree. */
+ * selects a variant for every call of the degree, with two exceptions: 0 ends
+ * a selection, so that calls take theirs by their number of limbs again (the
+ * degree's last variant is variant 0 for every call), and the tuner's last
+ * choice is selected as the tuner does.  Selecting what yell_get_variant
+ * returned earlier (0: nothing was selected) thus restores the dispatch of that
+ * time.  yell_variant_for gives the variant that a transform, or with polymul
+ * != 0 a fused polymul, of so many limbs (count * L) runs now. */
 int yell_variant_count(uint32_t log_n, uint32_t* count);
 int yell_variant_name(uint32_t log_n, uint32_t variant, char* buf, size_t len);
 int yell_set_variant(uint32_t log_n, uint32_t variant);
 int yell_get_variant(uint32_t log_n, uint32_t* variant);
+int yell_variant_for(uint32_t log_n, uint32_t limbs, int polymul, uint32_t* variant);
 int yell_autotune(uint32_t log_n, uint32_t L, uint32_t pairs, uint32_t* best, double* best_ms);
 
 /* Integer roofline (no counterpart in the reference): runs the production CT

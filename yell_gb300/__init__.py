@@ -365,12 +365,21 @@ def variants(log_n: int) -> list[str]:
 
 
 def set_variant(log_n: int, v: int) -> None:
+    """Selects a variant for every call of the degree; 0 ends a selection (the last
+    variant is variant 0 for every call), and what get_variant returned restores it."""
     call("yell_set_variant", log_n, v)
 
 
 def get_variant(log_n: int) -> int:
     v = ctypes.c_uint32()
     call("yell_get_variant", log_n, ctypes.addressof(v))
+    return v.value
+
+
+def variant_for(log_n: int, limbs: int, polymul: bool = False) -> int:
+    """The variant that a transform, or a fused polymul, of so many limbs runs now."""
+    v = ctypes.c_uint32()
+    call("yell_variant_for", log_n, limbs, int(polymul), ctypes.addressof(v))
     return v.value
 
 

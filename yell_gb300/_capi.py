@@ -147,6 +147,7 @@ SIGNATURES = {
     "yell_variant_name": (_int, [_u32, _u32, ctypes.c_char_p, _sz]),
     "yell_set_variant": (_int, [_u32, _u32]),
     "yell_get_variant": (_int, [_u32, _vp]),
+    "yell_variant_for": (_int, [_u32, _u32, _int, _vp]),
     "yell_autotune": (_int, [_u32, _u32, _u32, _vp, _vp]),
     "yell_server_create": (_int, [_vp, _vp]),
     "yell_server_destroy": (_int, [_vp]),

@@ -114,9 +114,9 @@ int num_sms() {
 std::vector<Variant> g_table[kMaxLogN + 1];
 std::once_flag g_table_once;
 // Selected variant + 1, with kTuned when the autotuner selected it, or 0 when
-// none was selected.
+// none was selected; and the tuner's last choice + 1, or 0.
 constexpr uint32_t kTuned = 0x80;
-std::array<std::array<std::atomic<uint8_t>, kMaxLogN + 1>, 64> g_selected{};
+std::array<std::array<std::atomic<uint8_t>, kMaxLogN + 1>, 64> g_selected{}, g_tuned{};
 
 void build_table() {
   add_whole_variants_small(g_table);
@@ -130,6 +130,12 @@ void build_table() {
   add_few_limb_variants(g_table);
   add_two_pass_few_variants(g_table);
   add_cluster_variants(g_table);
+  for (uint32_t n = kMinLogN; n <= kMaxLogN; ++n) {
+    Variant v = g_table[n][0];
+    v.again = true;
+    std::strncat(v.name, ", for every call", sizeof(v.name) - std::strlen(v.name) - 1);
+    g_table[n].push_back(v);
+  }
 }
 
 int current_device() {
@@ -138,12 +144,15 @@ int current_device() {
   return (d >= 0 && d < 64) ? d : 0;
 }
 
+}  // namespace
+
 // The variant a call of `limbs` limbs runs: the selected one, else the one
 // registered for that many limbs, else the first.  A variant that the
 // autotuner selected takes the first one's place, behind those for few limbs:
 // it was timed at one size (2^14 tuned at 32 limbs picked 4 words per thread,
 // at which an NTT of 512 limbs took 99 us against 77).
-const Variant& pick(uint32_t log_n, uint32_t limbs, LimbRange (Variant::*ranges)[2]) {
+const Variant& variant_for(uint32_t log_n, uint32_t limbs, bool polymul) {
+  LimbRange(Variant::*const ranges)[2] = polymul ? &Variant::polymul_at : &Variant::ntt_at;
   const std::vector<Variant>& vs = variants_of(log_n);
   const uint32_t sel = g_selected[current_device()][log_n].load(std::memory_order_relaxed);
   const bool tuned = (sel & kTuned) != 0;
@@ -159,8 +168,6 @@ const Variant& pick(uint32_t log_n, uint32_t limbs, LimbRange (Variant::*ranges)
   return *best;
 }
 
-}  // namespace
-
 const std::vector<Variant>& variants_of(uint32_t log_n) {
   std::call_once(g_table_once, build_table);
   return g_table[log_n];
@@ -171,8 +178,15 @@ uint32_t selected_variant(int device, uint32_t log_n) {
   return sel != 0 ? (sel & ~kTuned) - 1 : 0;
 }
 
-void select_variant(int device, uint32_t log_n, uint32_t v, bool tuned) {
-  g_selected[device][log_n].store((uint8_t)((v + 1) | (tuned ? kTuned : 0)), std::memory_order_relaxed);
+void select_tuned_variant(int device, uint32_t log_n, uint32_t v) {
+  g_tuned[device][log_n].store((uint8_t)(v + 1), std::memory_order_relaxed);
+  g_selected[device][log_n].store((uint8_t)((v + 1) | kTuned), std::memory_order_relaxed);
+}
+
+void select_variant(int device, uint32_t log_n, uint32_t v) {
+  uint32_t sel = v != 0 ? v + 1 : 0;
+  if (g_tuned[device][log_n].load(std::memory_order_relaxed) == v + 1) sel = (v + 1) | kTuned;
+  g_selected[device][log_n].store((uint8_t)sel, std::memory_order_relaxed);
 }
 
 cudaError_t init_kernel_attributes() {
@@ -212,7 +226,7 @@ cudaError_t launch_ntt(const LimbSet& ls, uint32_t log_n, const DevMod* mods, Nt
                        const NttShape&, cudaStream_t st) {
   if (ls.count == 0) return cudaSuccess;
   if (log_n < kMinLogN || log_n > kMaxLogN) return cudaErrorInvalidValue;
-  return pick(log_n, ls.count, &Variant::ntt_at).ntt(ls, mods, dir, st);
+  return variant_for(log_n, ls.count, false).ntt(ls, mods, dir, st);
 }
 
 cudaError_t launch_polymul(const LimbSet& c, const ConstLimbSet& a, const ConstLimbSet& b,
@@ -220,7 +234,7 @@ cudaError_t launch_polymul(const LimbSet& c, const ConstLimbSet& a, const ConstL
                            const NttShape&, cudaStream_t st, uint64_t* const* scratch_ptrs) {
   if (c.count == 0) return cudaSuccess;
   if (log_n < kMinLogN || log_n > kMaxLogN) return cudaErrorInvalidValue;
-  const Variant* v = &pick(log_n, c.count, &Variant::polymul_at);
+  const Variant* v = &variant_for(log_n, c.count, true);
   if (v->polymul_scratch && scratch == nullptr && scratch_ptrs == nullptr) {
     // Without scratch, the first (selection order) variant that needs none.
     v = nullptr;

@@ -5,12 +5,13 @@
 // the tile size of the whole-limb path (limbs per CTA) or the number of
 // column stages k1 of the two-pass path (columns of 2^k1 words, rows of
 // 2^(log_n - k1) words), or one limb per thread-block cluster.  A degree for
-// which no variant was selected takes the one registered for the call's
-// number of limbs (polymul_at, ntt_at), else variant 0; the autotuner
-// times every variant of a degree but those for few limbs on the current
-// device and selects the fastest, which then runs at every number of limbs
-// that no variant for few limbs is registered for.  A variant selected by
-// hand runs at every number of limbs.
+// which no variant was selected, or variant 0 was, takes the one registered
+// for the call's number of limbs (polymul_at, ntt_at), else variant 0; the
+// autotuner times every variant of a degree but those for few limbs on the
+// current device and selects the fastest, which then runs at every number of
+// limbs that no variant for few limbs is registered for.  Another variant
+// selected by hand runs at every number of limbs; the last of each degree is
+// variant 0 once more, for that.
 #pragma once
 #include <vector>
 
@@ -37,6 +38,8 @@ struct Variant {
   // One of the variants for few limbs: never the stand-in for a polymul
   // called without scratch.
   bool few_limbs = false;
+  // Variant 0 once more: selected, it runs at every number of limbs.
+  bool again = false;
 };
 
 constexpr uint32_t kAnyLimbs = 0xFFFFFFFFu;
@@ -66,10 +69,17 @@ void add_few_limb_variants(std::vector<Variant>* by_degree);     // 2^6 .. 2^10,
 void add_two_pass_few_variants(std::vector<Variant>* by_degree); // 2^13 .. 2^20, small tiles
 void add_cluster_variants(std::vector<Variant>* by_degree);      // 2^10 .. 2^14, one limb per cluster
 
-// Variant table of a degree, and the variant selected on the current device.
+// Variant table of a degree.
 const std::vector<Variant>& variants_of(uint32_t log_n);
-// (0 when none was).
+// The variant selected on a device (0 when none was), and its selection by the
+// autotuner or by hand.  By hand, 0 ends a selection, and the tuner's last
+// choice stands as if the tuner had selected it: selecting what
+// selected_variant returned earlier restores the dispatch of that time.
 uint32_t selected_variant(int device, uint32_t log_n);
-void select_variant(int device, uint32_t log_n, uint32_t v, bool tuned);
+void select_tuned_variant(int device, uint32_t log_n, uint32_t v);
+void select_variant(int device, uint32_t log_n, uint32_t v);
+// The variant that a transform (polymul: a fused polymul with scratch) of so
+// many limbs runs on the current device.
+const Variant& variant_for(uint32_t log_n, uint32_t limbs, bool polymul);
 
 }  // namespace yell_gb300

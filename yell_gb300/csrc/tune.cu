@@ -66,7 +66,10 @@ void load_tuning(int dev) {
     if (log_n < kMinLogN || log_n > kMaxLogN) continue;
     const std::vector<Variant>& vs = variants_of(log_n);
     for (uint32_t v = 0; v < vs.size(); ++v)
-      if (vname == vs[v].name) select_variant(dev, log_n, v, !vs[v].few_limbs);
+      if (vname == vs[v].name) {
+        if (vs[v].few_limbs || vs[v].again) select_variant(dev, log_n, v);
+        else select_tuned_variant(dev, log_n, v);
+      }
   }
 }
 
@@ -98,7 +101,7 @@ int yell_set_variant(uint32_t log_n, uint32_t variant) {
   if (variant >= variants_of(log_n).size()) return fail(kInvalidArgument, "no such variant");
   DeviceContext* ctx = DeviceContext::current(&st);
   if (!ctx) return st;
-  select_variant(ctx->device(), log_n, variant, false);
+  select_variant(ctx->device(), log_n, variant);
   return kOk;
 }
 
@@ -109,6 +112,14 @@ int yell_get_variant(uint32_t log_n, uint32_t* variant) {
   DeviceContext* ctx = DeviceContext::current(&st);
   if (!ctx) return st;
   *variant = selected_variant(ctx->device(), log_n);
+  return kOk;
+}
+
+int yell_variant_for(uint32_t log_n, uint32_t limbs, int polymul, uint32_t* variant) {
+  if (!variant || limbs == 0) return fail(kInvalidArgument, "null output or zero limbs");
+  const int st = check_degree(log_n);
+  if (st != kOk) return st;
+  *variant = (uint32_t)(&variant_for(log_n, limbs, polymul != 0) - variants_of(log_n).data());
   return kOk;
 }
 
@@ -143,7 +154,7 @@ int yell_autotune(uint32_t log_n, uint32_t L, uint32_t pairs, uint32_t* best, do
   uint32_t best_v = 0;
   double best_t = 1e30;
   for (uint32_t v = 0; v < vs.size() && e == cudaSuccess; ++v) {
-    if (vs[v].few_limbs) continue;  // chosen by a call's number of limbs
+    if (vs[v].few_limbs || vs[v].again) continue;  // chosen by a call's number of limbs; timed as variant 0
     float t = 1e30f;
     for (int rep = 0; rep < 4 && e == cudaSuccess; ++rep) {
       e = cudaEventRecord(e0, s);
@@ -163,7 +174,7 @@ int yell_autotune(uint32_t log_n, uint32_t L, uint32_t pairs, uint32_t* best, do
   cudaEventDestroy(e1);
   cudaFree(buf);
   if (e != cudaSuccess) return fail_cuda(e, "autotune run");
-  select_variant(ctx->device(), log_n, best_v, true);
+  select_tuned_variant(ctx->device(), log_n, best_v);
   persist(ctx->device(), log_n, vs[best_v].name);
   if (best) *best = best_v;
   if (best_ms) *best_ms = best_t;
