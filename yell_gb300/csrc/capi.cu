@@ -75,6 +75,13 @@ int check_aligned(const void* p, const char* what) {
 // pageable (pinned memory copies as fast by DMA) and 16-byte aligned.
 bool direct_host(DeviceContext* ctx, const void* p) { return ctx->host_access() && pageable_host(p); }
 
+// Degrees whose small calls run on the mapped host buffer when they are one
+// launch.  All of these have a polymul without scratch.  Above, two limbs
+// already run faster through device memory (GB300, 2 limbs of 2^14, us, mapped
+// and through the device: polymul 63 and 48, transform 34 and 27; 4 limbs of
+// 2^13, the same words: 59 and 36 mapped).
+constexpr uint32_t kSmallCallLogN = 13;
+
 // Host-memory drop-in: copy L limbs (separate host arrays) into the context's
 // staging area, run `body`, copy `nout` result limb sets back, synchronise.
 // Holds the staging lock for the whole call.
@@ -90,8 +97,8 @@ int host_ntt(uint64_t* const* limbs, uint32_t L, uint32_t log_n, uint32_t cm0, N
   YELL_TRY(ctx->ensure_tables(log_n, cm0, L, &mods));
   const size_t n = (size_t)1 << log_n;
   cudaStream_t st = ctx->stream();
-  if (n * L <= DeviceContext::kSmallCallWords && ntt_launch_count(log_n, ctx->shape) == 1) {
-    // small call: one whole-limb launch in place on the mapped host buffer
+  if (log_n <= kSmallCallLogN && n * L <= DeviceContext::kSmallCallWords && ntt_launch_count(log_n, L) == 1) {
+    // small call: one launch in place on the mapped host buffer
     std::lock_guard<std::mutex> g(ctx->small.lock);
     YELL_TRY(ctx->small.ensure());
     for (uint32_t i = 0; i < L; ++i) std::memcpy(ctx->small.host + i * n, limbs[i], n * 8);
@@ -328,9 +335,9 @@ int yell_polymul_host(uint64_t* c, const uint64_t* a, const uint64_t* b, uint32_
   const DevMod* mods;
   YELL_TRY(ctx->ensure_tables(log_n, cm0, L, &mods));
   const size_t pair_words = ((size_t)L) << log_n;
-  if ((size_t)pairs * pair_words <= DeviceContext::kSmallCallWords &&
-      polymul_launch_count(log_n, ctx->shape) == 1) {
-    // small call: one whole-limb launch on the mapped host buffer
+  if (log_n <= kSmallCallLogN && (size_t)pairs * pair_words <= DeviceContext::kSmallCallWords &&
+      polymul_launch_count(log_n, pairs * L) == 1) {
+    // small call: one launch on the mapped host buffer
     const size_t w = (size_t)pairs * pair_words;
     std::lock_guard<std::mutex> g(ctx->small.lock);
     YELL_TRY(ctx->small.ensure());

@@ -163,8 +163,9 @@ cudaError_t gather_host_contiguous(uint64_t* dev, const uint64_t* host, uint32_t
 cudaError_t scatter_host_contiguous(uint64_t* host, const uint64_t* dev, uint32_t limbs, uint32_t log_n,
                                     cudaStream_t st);
 
-// Kernels launched by one call of launch_ntt / launch_polymul / elementwise.
-uint32_t ntt_launch_count(uint32_t log_n, const NttShape& shape);
-uint32_t polymul_launch_count(uint32_t log_n, const NttShape& shape);
+// Kernels launched by one call of launch_ntt / launch_polymul (with scratch)
+// of so many limbs, as the dispatch stands now.
+uint32_t ntt_launch_count(uint32_t log_n, uint32_t limbs);
+uint32_t polymul_launch_count(uint32_t log_n, uint32_t limbs);
 
 }  // namespace yell_gb300

@@ -198,11 +198,9 @@ cudaError_t init_kernel_attributes() {
   return cudaSuccess;
 }
 
-uint32_t ntt_launch_count(uint32_t log_n, const NttShape&) {
-  return variants_of(log_n)[selected_variant(current_device(), log_n)].ntt_launches;
-}
-uint32_t polymul_launch_count(uint32_t log_n, const NttShape&) {
-  return variants_of(log_n)[selected_variant(current_device(), log_n)].polymul_launches;
+uint32_t ntt_launch_count(uint32_t log_n, uint32_t limbs) { return variant_for(log_n, limbs, false).ntt_launches; }
+uint32_t polymul_launch_count(uint32_t log_n, uint32_t limbs) {
+  return variant_for(log_n, limbs, true).polymul_launches;
 }
 
 // The words a polymul of this degree may need, whichever variant is selected
