@@ -313,6 +313,7 @@ Variant cluster_variant() {
   v.set_attrs = &set_attrs_cluster<CC>;
   v.ntt_launches = 1;
   v.polymul_launches = 1;
+  v.tile_log = CC::T;
   return v;
 }
 

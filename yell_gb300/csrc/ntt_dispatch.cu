@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "kernels.h"
+#include "launch_size.h"
 #include "ntt_variants.h"
 #include "profiler.h"
 #include "runtime.h"
@@ -224,7 +225,9 @@ cudaError_t launch_ntt(const LimbSet& ls, uint32_t log_n, const DevMod* mods, Nt
                        const NttShape&, cudaStream_t st) {
   if (ls.count == 0) return cudaSuccess;
   if (log_n < kMinLogN || log_n > kMaxLogN) return cudaErrorInvalidValue;
-  return variant_for(log_n, ls.count, false).ntt(ls, mods, dir, st);
+  const Variant& v = variant_for(log_n, ls.count, false);
+  if (!one_launch(ls.count, log_n, v.tile_log)) return cudaErrorInvalidConfiguration;
+  return v.ntt(ls, mods, dir, st);
 }
 
 cudaError_t launch_polymul(const LimbSet& c, const ConstLimbSet& a, const ConstLimbSet& b,
@@ -243,6 +246,7 @@ cudaError_t launch_polymul(const LimbSet& c, const ConstLimbSet& a, const ConstL
       }
     if (!v) return cudaErrorInvalidValue;
   }
+  if (!one_launch(c.count, log_n, v->tile_log)) return cudaErrorInvalidConfiguration;
   return v->polymul(c, a, b, mods, scratch, scratch_ptrs, st);
 }
 

@@ -20,6 +20,7 @@
 // column tile); the other ends are staged through shared memory so that the
 // HBM accesses stay coalesced.
 #pragma once
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <type_traits>
@@ -1293,6 +1294,7 @@ Variant whole_variant() {
   v.set_attrs = &set_attrs_whole<LOGN, T, LOGE>;
   v.ntt_launches = 1;
   v.polymul_launches = 1;
+  v.tile_log = T;
   return v;
 }
 
@@ -1306,6 +1308,9 @@ Variant two_pass_of() {
   v.set_attrs = &set_attrs_two_pass<LOGN, K1, TT>;
   v.ntt_launches = 2;
   v.polymul_launches = 3;
+  v.tile_log = std::min({TT::Col2::T, TT::Rows::T, TT::ColFwd::T, TT::ColInv::T, TT::RowFwd::T, TT::RowInv::T});
+  if constexpr (!std::is_void_v<typename TT::RowFwd2>)
+    v.tile_log = std::min<uint32_t>(v.tile_log, std::min(TT::RowFwd2::T, TT::RowInv2::T));
   v.polymul_scratch = true;
   return v;
 }

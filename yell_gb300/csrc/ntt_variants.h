@@ -31,6 +31,7 @@ struct Variant {
   cudaError_t (*set_attrs)() = nullptr;
   uint32_t ntt_launches = 0;
   uint32_t polymul_launches = 0;
+  uint32_t tile_log = 0;  // log2 of the words of its smallest tile (words per CTA)
   bool polymul_scratch = false;  // the polymul needs one operand's worth of scratch words
   // Chosen without a selection for calls whose number of limbs lies in one of
   // these ranges; among several variants, the one whose range ends first.

@@ -95,8 +95,8 @@ int check_moduli(uint32_t cm0, uint32_t L) {
 int check_limbs(uint64_t count, uint32_t L, uint32_t log_n, uint32_t* limbs) {
   if (count == 0) return fail(kInvalidArgument, "zero polys or pairs");
   const uint64_t total = count * (uint64_t)L;  // count < 2^32, L <= kMaxModuli: no wrap
-  // One launch covers every limb: the grid (limbs, or 4096-word tiles of
-  // larger limbs) must stay below 2^31 blocks.
+  // Limbs, and 4096-word tiles of larger limbs, below 2^31.  What a launch
+  // takes depends on its kernel's tiles and is checked there (launch_size.h).
   const uint32_t shift = log_n > 12 ? log_n - 12 : 0;
   const uint64_t max_limbs = ((uint64_t(1) << 31) - 1) >> shift;
   if (total > max_limbs)
