@@ -15,6 +15,8 @@
 // (kCluster32).  The butterflies, their order and their twiddle indices are
 // the reference's, so lazy words match it exactly.
 #include <algorithm>
+#include <array>
+#include <atomic>
 #include <cstring>
 #include <memory>
 #include <mutex>
@@ -609,6 +611,8 @@ __global__ void k32_elementwise(uint32_t* dst, const uint32_t* a, const uint32_t
 
 // ---- launch ----------------------------------------------------------------------
 // Degrees of the one-CTA kernels; larger ones run on clusters only.
+// At 2^13 clusters take every inverse and polymul where one of 2 can be placed
+// (512 limbs, us: polymul 39.6 and 47.3 with one CTA, inverse 16.7 and 17.6).
 constexpr int kLogMaxOneCta32 = 13;
 // Host-pointer calls up to this degree run in place on the context's pinned,
 // device-mapped host buffer.
@@ -619,12 +623,9 @@ cudaError_t set_attrs32() {
   using C = typename Cfg32<LOGN>::C;
   const int smem = (int)Cfg32<LOGN>::kSmem;
   cudaError_t e = cudaSuccess;
-  for (auto k : {k32_ntt<C, 0>, k32_ntt<C, 1>})
+  for (auto k : {k32_ntt<C, 0>, k32_ntt<C, 1>, k32_ntt<C, 2>})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if constexpr (LOGN < kLogMaxOneCta32) {
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k32_ntt<C, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k32_polymul<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  }
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k32_polymul<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   return e;
 }
 
@@ -639,10 +640,8 @@ cudaError_t launch32(int kind, uint32_t* c, const uint32_t* a, const uint32_t* b
   const uint32_t blocks = (ls.count + (1u << (C::T - LOGN)) - 1) >> (C::T - LOGN);
   if (kind == 0) launch_dependent(k32_ntt<C, 0>, blocks, C::THREADS, CF::kSmem, st, c, ls, mods);
   else if (kind == 1) launch_dependent(k32_ntt<C, 1>, blocks, C::THREADS, CF::kSmem, st, c, ls, mods);
-  if constexpr (LOGN < kLogMaxOneCta32) {  // at 2^13 clusters take every inverse and polymul
-    if (kind == 2) launch_dependent(k32_ntt<C, 2>, blocks, C::THREADS, CF::kSmem, st, c, ls, mods);
-    else if (kind == 3) launch_dependent(k32_polymul<C>, blocks, C::THREADS, CF::kSmem, st, c, a, b, ls, mods + kMaxModuli32);
-  }
+  else if (kind == 2) launch_dependent(k32_ntt<C, 2>, blocks, C::THREADS, CF::kSmem, st, c, ls, mods);
+  else launch_dependent(k32_polymul<C>, blocks, C::THREADS, CF::kSmem, st, c, a, b, ls, mods + kMaxModuli32);
   return cudaGetLastError();
 }
 
@@ -696,6 +695,19 @@ cudaError_t staged_polymul32(uint32_t* c, const uint32_t* a, const uint32_t* b, 
   return cudaGetLastError();
 }
 cudaError_t attrs_staged32() { return set_smem(k32_polymul_staged, Staged32::kSmem); }
+// Cluster of 2 (compiled into the kernel), as ClusterCfg names it.
+struct StagedPair {
+  static constexpr int CL = 1, THREADS = Staged32::THREADS;
+};
+template <class CC>
+bool placeable_ntt32() {
+  return cluster_placeable<CC>(k_ntt_cluster<CC, 0, Out32, DevMod32>, 2 * CC::kTileBytes);
+}
+template <class CC>
+bool placeable_polymul32() {
+  return cluster_placeable<CC>(k_polymul_cluster<CC, Out32, In32, DevMod32>, 4 * CC::kTileBytes);
+}
+bool placeable_staged32() { return cluster_placeable<StagedPair>(k32_polymul_staged, Staged32::kSmem); }
 
 // Cluster kernels (one limb per cluster of 2^CL CTAs) by degree and number of
 // limbs: a call takes the entry of its degree with the smallest bound that
@@ -723,16 +735,18 @@ struct Cluster32 {
   cudaError_t (*polymul)(uint32_t*, const uint32_t*, const uint32_t*, const Limbs32&, const DevMod32*, cudaStream_t);
   cudaError_t (*ntt_attrs)();
   cudaError_t (*polymul_attrs)();
+  bool (*placeable)();  // on the current device
 };
 template <int LOGN, int K1, int LOGE, int CL, int PB = 0>
 using CC32 = ClusterCfg<LOGN, K1, LOGE, CL, uint32_t, PB>;
 template <class CC>
 constexpr Cluster32 polymul_route32(uint32_t upto) {
-  return {CC::LOGN, upto, 0, 0, nullptr, cluster_polymul32<CC>, nullptr, attrs_polymul32<CC>};
+  return {CC::LOGN, upto, 0, 0, nullptr, cluster_polymul32<CC>, nullptr, attrs_polymul32<CC>,
+          placeable_polymul32<CC>};
 }
 template <class CC>
 constexpr Cluster32 ntt_route32(uint32_t fwd, uint32_t inv) {
-  return {CC::LOGN, 0, fwd, inv, cluster_ntt32<CC>, nullptr, attrs_ntt32<CC>, nullptr};
+  return {CC::LOGN, 0, fwd, inv, cluster_ntt32<CC>, nullptr, attrs_ntt32<CC>, nullptr, placeable_ntt32<CC>};
 }
 constexpr uint32_t kAny32 = 0xFFFFFFFFu;
 constexpr Cluster32 kCluster32[] = {
@@ -754,17 +768,30 @@ constexpr Cluster32 kCluster32[] = {
     ntt_route32<CC32<14, 7, 4, 2>>(kAny32, kAny32),
     polymul_route32<CC32<15, 8, 4, 3, 2>>(32),
     polymul_route32<CC32<15, 8, 4, 3, 3>>(57),
-    {15, 76, 0, 0, nullptr, staged_polymul32, nullptr, attrs_staged32},
+    {15, 76, 0, 0, nullptr, staged_polymul32, nullptr, attrs_staged32, placeable_staged32},
     polymul_route32<CC32<15, 8, 4, 3, 3>>(kAny32),
     ntt_route32<CC32<15, 8, 4, 3>>(kAny32, kAny32),
+    // where no clusters of 4 or 8 can be placed (GB300, 512 limbs, us, the
+    // entries above -> these, polymul / forward / inverse: 2^14 86 -> 104 / 34 ->
+    // 37 / 32 -> 33; 2^15 187 -> 199 / 71 -> 90 / 65 -> 81)
+    polymul_route32<CC32<14, 7, 4, 1>>(kAny32),
+    ntt_route32<CC32<14, 7, 4, 1>>(kAny32, kAny32),
+    {15, kAny32, 0, 0, nullptr, staged_polymul32, nullptr, nullptr, placeable_staged32},
+    ntt_route32<CC32<15, 8, 4, 1>>(kAny32, kAny32),
 };
+constexpr size_t kRoutes32 = sizeof(kCluster32) / sizeof(kCluster32[0]);
+// Per device, the entries whose clusters it can place, one bit each.
+std::array<std::atomic<uint64_t>, 64> g_placeable32{};
+static_assert(kRoutes32 <= 64, "a bit per entry");
 
-// The entry of kCluster32 for a call, or nullptr.
-const Cluster32* route32(uint32_t log_n, int kind, uint32_t limbs) {
+// The entry of kCluster32 for a call, the first of those with the same bound,
+// or nullptr.
+const Cluster32* route32(int device, uint32_t log_n, int kind, uint32_t limbs) {
+  const uint64_t placeable = g_placeable32[device].load(std::memory_order_relaxed);
   const auto bound = kind == 3 ? &Cluster32::polymul_upto : (kind == 2 ? &Cluster32::inv_upto : &Cluster32::fwd_upto);
   const Cluster32* best = nullptr;
   for (const Cluster32& r : kCluster32)
-    if (r.log_n == log_n && r.*bound >= limbs && (!best || r.*bound < best->*bound)) best = &r;
+    if (r.log_n == log_n && (placeable >> (&r - kCluster32) & 1) && r.*bound >= limbs && (!best || r.*bound < best->*bound)) best = &r;
   return best;
 }
 
@@ -805,6 +832,10 @@ int prepare32(uint32_t log_n, uint32_t cm0, uint32_t L, DeviceContext** ctx, con
         if (e == cudaSuccess && r.ntt_attrs) e = r.ntt_attrs();
         if (e == cudaSuccess && r.polymul_attrs) e = r.polymul_attrs();
       }
+      uint64_t placeable = 0;
+      for (size_t i = 0; i < kRoutes32 && e == cudaSuccess; ++i)
+        if (kCluster32[i].placeable()) placeable |= uint64_t(1) << i;
+      g_placeable32[dev].store(placeable, std::memory_order_relaxed);
       if (e != cudaSuccess) return fail_cuda(e, "32-bit kernel attributes");
       done.push_back(dev);
     }
@@ -832,7 +863,7 @@ int run32(int kind, uint32_t* c, const uint32_t* a, const uint32_t* b, uint32_t 
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->stream();
   static const char* names[4] = {"ntt32_forward", "ntt32_forward_lazy", "ntt32_backward", "polymul32"};
   LaunchScope ps(names[kind], s);
-  const Cluster32* r = route32(log_n, kind, ls.count);
+  const Cluster32* r = route32(ctx->device(), log_n, kind, ls.count);
   const cudaError_t e = !r ? dispatch32(OneCta32{}, log_n, kind, c, a, b, ls, mods, s)
                         : kind == 3 ? r->polymul(c, a, b, ls, mods, s)
                                     : r->ntt(kind, c, ls, mods, s);

@@ -19,6 +19,8 @@
 // barriers; once the limbs fill the chip, the 64-bit multiplier, where the
 // 16-word tiles win because they exchange less (the bounds in ntt_cluster.cu).
 #pragma once
+#include <cstdlib>
+
 #include "ntt_kernels.cuh"
 
 namespace yell_gb300 {
@@ -247,6 +249,32 @@ __global__ void __launch_bounds__(CC::THREADS, CC::kPolymulBlocks)
   gstore_cols<C0, CC::LOGB>(xa, c.limb(limb, log_n) + (rank << CC::LB), c0);
 }
 
+// Whether the current device can place a cluster of the kernel's CTAs: a small
+// partition may have no 8 SMs side by side.  YELL_GB300_MAX_CLUSTER bounds the
+// clusters of a process that shares its device with other work.
+template <class CC, typename... KArgs>
+bool cluster_placeable(void (*kernel)(KArgs...), size_t smem) {
+  const char* bound = std::getenv("YELL_GB300_MAX_CLUSTER");
+  if (bound && *bound && std::atoi(bound) < (1 << CC::CL)) return false;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1u << CC::CL;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1u << CC::CL);
+  cfg.blockDim = dim3(CC::THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return clusters > 0;
+}
+
 // Launch of a cluster kernel, as a programmatic dependent like the two-pass
 // kernels.
 template <class CC, typename... KArgs, typename... Args>
@@ -302,6 +330,12 @@ cudaError_t set_attrs_cluster() {
   return set_smem(k_polymul_cluster<CC, LimbSet, ConstLimbSet, DevMod>, polymul);
 }
 
+template <class CC>
+bool cluster_variant_placeable() {
+  return cluster_placeable<CC>(k_ntt_cluster<CC, 0, LimbSet, DevMod>, 2 * CC::kTileBytes) &&
+         cluster_placeable<CC>(k_polymul_cluster<CC, LimbSet, ConstLimbSet, DevMod>, 4 * CC::kTileBytes);
+}
+
 template <int LOGN, int K1, int LOGE, int CL>
 Variant cluster_variant() {
   using CC = ClusterCfg<LOGN, K1, LOGE, CL>;
@@ -311,6 +345,7 @@ Variant cluster_variant() {
   v.ntt = &launch_cluster_ntt<CC>;
   v.polymul = &launch_cluster_polymul<CC>;
   v.set_attrs = &set_attrs_cluster<CC>;
+  v.placeable = &cluster_variant_placeable<CC>;
   v.ntt_launches = 1;
   v.polymul_launches = 1;
   v.tile_log = CC::T;

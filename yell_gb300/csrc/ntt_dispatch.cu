@@ -119,6 +119,10 @@ std::once_flag g_table_once;
 constexpr uint32_t kTuned = 0x80;
 std::array<std::array<std::atomic<uint8_t>, kMaxLogN + 1>, 64> g_selected{}, g_tuned{};
 
+// Variants whose clusters the device cannot place, one bit each: never taken
+// for a call's number of limbs (selected by hand, their launch fails).
+std::array<std::array<std::atomic<uint64_t>, kMaxLogN + 1>, 64> g_unplaceable{};
+
 void build_table() {
   add_whole_variants_small(g_table);
   add_whole_variants_large(g_table);
@@ -155,14 +159,17 @@ int current_device() {
 const Variant& variant_for(uint32_t log_n, uint32_t limbs, bool polymul) {
   LimbRange(Variant::*const ranges)[2] = polymul ? &Variant::polymul_at : &Variant::ntt_at;
   const std::vector<Variant>& vs = variants_of(log_n);
-  const uint32_t sel = g_selected[current_device()][log_n].load(std::memory_order_relaxed);
+  const int dev = current_device();
+  const uint32_t sel = g_selected[dev][log_n].load(std::memory_order_relaxed);
+  const uint64_t unplaceable = g_unplaceable[dev][log_n].load(std::memory_order_relaxed);
   const bool tuned = (sel & kTuned) != 0;
   if (sel != 0 && !tuned) return vs[sel - 1];
   const Variant* best = &vs[tuned ? (sel & ~kTuned) - 1 : 0];
   uint64_t most = ~0ull;
   for (const Variant& v : vs)
     for (const LimbRange& r : v.*ranges)
-      if ((!tuned || v.few_limbs) && r.least <= limbs && limbs <= r.most && r.most < most) {
+      if ((!tuned || v.few_limbs) && r.least <= limbs && limbs <= r.most && r.most < most &&
+          !(unplaceable >> (&v - vs.data()) & 1)) {
         best = &v;
         most = r.most;
       }
@@ -191,11 +198,16 @@ void select_variant(int device, uint32_t log_n, uint32_t v) {
 }
 
 cudaError_t init_kernel_attributes() {
-  for (uint32_t n = kMinLogN; n <= kMaxLogN; ++n)
+  const int dev = current_device();
+  for (uint32_t n = kMinLogN; n <= kMaxLogN; ++n) {
+    uint64_t unplaceable = 0;
     for (const Variant& v : variants_of(n)) {
       const cudaError_t e = v.set_attrs();
       if (e != cudaSuccess) return e;
+      if (v.placeable && !v.placeable()) unplaceable |= uint64_t(1) << (&v - variants_of(n).data());
     }
+    g_unplaceable[dev][n].store(unplaceable, std::memory_order_relaxed);
+  }
   return cudaSuccess;
 }
 

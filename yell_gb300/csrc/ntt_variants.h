@@ -29,6 +29,9 @@ struct Variant {
   cudaError_t (*polymul)(const LimbSet&, const ConstLimbSet&, const ConstLimbSet&, const DevMod*,
                          uint64_t* scratch, uint64_t* const* scratch_ptrs, cudaStream_t) = nullptr;
   cudaError_t (*set_attrs)() = nullptr;
+  // Whether the current device can place the kernels' clusters (nullptr: no
+  // clusters).  Asked once per device, after set_attrs.
+  bool (*placeable)() = nullptr;
   uint32_t ntt_launches = 0;
   uint32_t polymul_launches = 0;
   uint32_t tile_log = 0;  // log2 of the words of its smallest tile (words per CTA)
