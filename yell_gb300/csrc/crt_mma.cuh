@@ -203,7 +203,7 @@ __global__ void k_crt_wait_check(uint32_t limit, uint32_t* status) {
 // image: image_bytes(L, N) bytes in operand layout; mods: L entries.
 template <uint32_t NC>  // chunks(L)
 __global__ void __launch_bounds__(kThreads, 1)
-    k_crt_mma(uint64_t* __restrict__ out, const uint64_t* __restrict__ in, uint64_t coeffs, uint32_t L, uint32_t log_n,
+    k_crt_mma(uint64_t* out, const uint64_t* in, uint64_t coeffs, uint32_t L, uint32_t log_n,
               const Mod* __restrict__ mods, const uint4* __restrict__ image, const uint64_t* __restrict__ qw,
               uint32_t W, uint32_t* status) {
   extern __shared__ uint8_t smem_raw[];
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     auto fetch = [&](uint32_t c) {
 #pragma unroll
       for (int i = 0; i < (int)kMine; ++i)
-        r[c][i] = live && (c + 1 < NC || i < last) ? __ldg(src + i * n) : 0;
+        r[c][i] = live && (c + 1 < NC || i < last) ? src[i * n] : 0;
       src += kChunkMods * n;
     };
     locate(blockIdx.x);

@@ -244,7 +244,7 @@ __device__ __forceinline__ void stage_in32(uint32_t* s, const uint32_t* g, uint3
     const uint32_t v = (threadIdx.x + i * C::THREADS) * 4;
     const uint32_t limb = limb0 + (v >> C::K);
     if (limb < count)
-      d[i] = __ldg(reinterpret_cast<const uint4*>(g + ((size_t)limb << C::K) + (v & ((1u << C::K) - 1u))));
+      d[i] = *reinterpret_cast<const uint4*>(g + ((size_t)limb << C::K) + (v & ((1u << C::K) - 1u)));
   }
 #pragma unroll
   for (int i = 0; i < IT; ++i) {

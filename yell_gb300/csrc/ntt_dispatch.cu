@@ -22,8 +22,9 @@ namespace yell_gb300 {
 
 namespace {
 
+// plain, as in the transforms (ntt_kernels.cuh)
 __device__ __forceinline__ ulonglong2 ld_pair(const uint64_t* p) {
-  return __ldg(reinterpret_cast<const ulonglong2*>(p));
+  return *reinterpret_cast<const ulonglong2*>(p);
 }
 
 __device__ __forceinline__ void st_pair(uint64_t* p, uint64_t a, uint64_t b) {

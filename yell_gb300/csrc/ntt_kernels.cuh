@@ -40,12 +40,23 @@ namespace {
 
 constexpr int kTileLog = 12;  // 4096 words per two-pass tile
 
+// The caller's words, and those of a pass before.  The read-only path (__ldg)
+// is for memory that nobody writes while the kernel runs, and a kernel launched
+// as a dependent runs, waiting, beside the one that writes them; volatile keeps
+// the loads behind that wait.
 __device__ __forceinline__ ulonglong2 ld_pair(const uint64_t* p) {
-  return __ldg(reinterpret_cast<const ulonglong2*>(p));
+  ulonglong2 v;
+  asm volatile("ld.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint64_t ld_word(const uint64_t* p) {
+  uint64_t v;
+  asm volatile("ld.global.u64 %0, [%1];" : "=l"(v) : "l"(p));
+  return v;
 }
 
 // Loads of words another CTA of the same launch wrote (the persistent batch
-// kernel's intermediates): through L2, never the non-coherent read-only path.
+// kernel's intermediates): through L2.
 __device__ __forceinline__ ulonglong2 ld_pair_cg(const uint64_t* p) {
   ulonglong2 v;
   asm volatile("ld.global.cg.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p));
@@ -64,18 +75,18 @@ __device__ __forceinline__ ulonglong2 ld_pair_t(const uint64_t* p) {
 // 32-bit words (only the kernels without COH use them)
 template <bool COH>
 __device__ __forceinline__ uint2 ld_pair_t(const uint32_t* p) {
-  static_assert(!COH, "32-bit words are read through the read-only path");
-  return __ldg(reinterpret_cast<const uint2*>(p));
+  static_assert(!COH, "no 32-bit kernel reads words of its own launch");
+  return *reinterpret_cast<const uint2*>(p);
 }
 template <bool COH>
 __device__ __forceinline__ uint32_t ld_word_t(const uint32_t* p) {
-  static_assert(!COH, "32-bit words are read through the read-only path");
-  return __ldg(p);
+  static_assert(!COH, "no 32-bit kernel reads words of its own launch");
+  return *p;
 }
 template <bool COH>
 __device__ __forceinline__ uint64_t ld_word_t(const uint64_t* p) {
   if constexpr (COH) return ld_cg(p);
-  else return __ldg(p);
+  else return ld_word(p);
 }
 
 __device__ __forceinline__ void st_pair(uint64_t* p, uint64_t a, uint64_t b) {
@@ -104,7 +115,7 @@ __device__ __forceinline__ void gload_rows(W* x, const W* g, uint32_t base_u) {
   } else if constexpr (RG::CONTIG && sizeof(W) == 4 && R >= 2) {
 #pragma unroll
     for (int j = 0; j < (1 << R); j += 4) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(gb + j));
+      const uint4 v = *reinterpret_cast<const uint4*>(gb + j);
       x[j] = v.x;
       x[j + 1] = v.y;
       x[j + 2] = v.z;
@@ -426,8 +437,14 @@ __global__ void __launch_bounds__(C::THREADS, min_blocks(INV ? 1024 : 768, C::TH
   const uint32_t col0 = (blockIdx.x & ((1u << TPL) - 1u)) << LB;
   const uint64_t* in = src.limb(limb, log_n) + col0;
   uint64_t* out = dst.limb(limb, log_n) + col0;
-  const DevMod m = load_mod(mods, dst.cm(limb));
   uint64_t x[1 << C::LOGE];
+  // the inverse requests its words first: 512 limbs of 2^16 at k1 = 7 153.7 us
+  // against 161.5 with the constants first
+  if constexpr (INV) {
+    using RB = Round<C, NR - 1>;
+    gload_cols<RB, LOGB>(x, in, RB::base(tid));
+  }
+  const DevMod m = load_mod(mods, dst.cm(limb));
   if constexpr (!INV) {
     using R0 = Round<C, 0>;
     const uint32_t b0 = R0::base(tid);
@@ -448,7 +465,6 @@ __global__ void __launch_bounds__(C::THREADS, min_blocks(INV ? 1024 : 768, C::TH
   } else {
     using RB = Round<C, NR - 1>;  // bottom round, executed first
     const uint32_t bb = RB::base(tid);
-    gload_cols<RB, LOGB>(x, in, bb);
     if constexpr (NR == 1) {
       gs_round<RB, true>(x, log_n, LOGB + RB::BETA, RB::gr(bb, 0), m);
       gstore_cols<RB, LOGB>(x, out, bb);

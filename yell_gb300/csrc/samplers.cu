@@ -295,8 +295,8 @@ __global__ void __launch_bounds__(kRankThreads) k_hwt_rank(uint32_t* hitted, Hwt
 // Coefficient i of poly j: chosen when its bit is set; its sign is sign word
 // (signs start) + rank of the position of the poly's stream.
 __global__ void k_hwt_write(uint64_t* out, uint32_t count, uint32_t L, uint32_t log_n, uint32_t cm0,
-                            const DevMod* __restrict__ mods, uint64_t seed, uint32_t h, const HwtCtl* __restrict__ ctl,
-                            const uint32_t* __restrict__ bits, const uint32_t* __restrict__ prefix) {
+                            const DevMod* __restrict__ mods, uint64_t seed, uint32_t h, const HwtCtl* ctl,
+                            const uint32_t* bits, const uint32_t* prefix) {
   const size_t pairs = ((size_t)count << log_n) >> 1;
   const uint32_t nmask = (1u << log_n) - 1u;
   const uint32_t nw = log_n >= 5 ? 1u << (log_n - 5) : 1u;
@@ -306,15 +306,15 @@ __global__ void k_hwt_write(uint64_t* out, uint32_t count, uint32_t L, uint32_t 
     const size_t poly = k >> log_n;
     const uint32_t i = (uint32_t)k & nmask;  // even: i and i + 1 share a bit word
     const size_t wi = poly * nw + (i >> 5);
-    const uint32_t b = __ldg(&bits[wi]);
+    const uint32_t b = bits[wi];
     const uint32_t sh = i & 31u;
     const uint32_t b0 = (b >> sh) & 1u, b1 = (b >> (sh + 1)) & 1u;
     int64_t e0 = 0, e1 = 0;
     if (b0 | b1) {
       const uint64_t s = rand_word(seed, poly);
-      const uint32_t draws = __ldg(&ctl[poly].draws);
+      const uint32_t draws = ctl[poly].draws;
       const uint64_t signs = (uint64_t)((draws + h - 1) / h) * h;
-      const uint32_t rank0 = __ldg(&prefix[wi]) + __popc(b & ((1u << sh) - 1u));
+      const uint32_t rank0 = prefix[wi] + __popc(b & ((1u << sh) - 1u));
       if (b0) e0 = (rand_word(s, signs + rank0) & 2) ? 1 : -1;
       if (b1) e1 = (rand_word(s, signs + rank0 + b0) & 2) ? 1 : -1;
     }
