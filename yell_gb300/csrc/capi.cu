@@ -354,10 +354,11 @@ int yell_polymul_host(uint64_t* c, const uint64_t* a, const uint64_t* b, uint32_
   }
   // ~64 MiB of operands per chunk, at least one pair.  The last chunks are
   // smaller, so that the compute and the D2H left after the final H2D cover
-  // little, but not below 4 MiB per operand: a chunk's eleven calls take the
-  // host about 25 us, in which the link moves 5 MiB.  (GB300, 5 pairs of 8 x
-  // 2^15 words, 2 MiB each: one pair per chunk 230 us, two 182, of which the
-  // operands' transfer is 99; 8 pairs of 8 x 2^16, 4 MiB each: 499 and 498.)
+  // little, but units of at least 4 MiB per operand (and what remains): a
+  // chunk's eleven calls take the host about 25 us, in which the link moves 5
+  // MiB.  (GB300, 5 pairs of 8 x 2^15 words, 2 MiB each: one pair per chunk 230
+  // us, two, two and one 182, of which the operands' transfer is 99; 8 pairs of
+  // 8 x 2^16, 4 MiB each: 499 and 498.)
   const size_t target = (64ull << 20) / 8;
   uint32_t cp = (uint32_t)std::max<size_t>(1, target / (2 * pair_words));
   if (cp > pairs) cp = pairs;

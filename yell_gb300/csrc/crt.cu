@@ -459,8 +459,8 @@ int crt_lift(uint64_t* d_out, const uint64_t* d_in, uint32_t count, uint32_t L, 
   if (s != kOk) return s;
   // From 4 moduli up the tensor-core kernel is the faster one at every number
   // of coefficients (GB300, us, digit kernel -> tensor cores: 2^20
-  // coefficients, L = 3: 33 -> 41, 4: 53 -> 42, 8: 117 -> 48, 16: 286 -> 80,
-  // 32: 762 -> 143; 2^13, L = 3: 3.7 -> 4.1, 32: 35 -> 6); its digits are exact
+  // coefficients, L = 3: 33 -> 41, 4: 53 -> 38, 8: 117 -> 47, 16: 286 -> 78,
+  // 32: 762 -> 139; 2^13, L = 3: 3.7 -> 4.1, 32: 35 -> 6); its digits are exact
   // up to kMaxL moduli.
   if (t->image) {
     const cudaError_t me = launch_crt_mma(d_out, d_in, (uint64_t)count << log_n, L, log_n, t, st, device, own_status);

@@ -34,13 +34,14 @@
 // the carries while the other accumulator fills, and write the words through
 // shared memory in segments of 64 bytes.
 //
-// What bounds it: per tile at L = 32 the tensor cores need 2190 cycles, HBM
-// (63 words per coefficient) 3000, the 12 300 warp instructions of producers
-// and epilogue about 5000 at the SM's issue rate for this mix.  GB300, 16 x
-// 2^16 coefficients, L = 32: 143 us, 3.7 TB/s (762 us for the kernel with
-// 32-bit multiply-add chains).  On the way: one-lane issue loop 166 us, TMEM
-// loads of 32 columns two deep (spills) 339 us, producers' own proxy fences
-// 181 us.
+// What bounds it: no one unit.  Per tile at L = 32 the tensor cores need 2190
+// cycles, HBM (63 words per coefficient) 3000, and a tile takes about 5000;
+// the counters have issue slots at 48%, the tensor pipe at 37%, DRAM at 22%,
+// and warps waiting on long scoreboards, fixed latencies and the barriers
+// between them.  GB300, 16 x 2^16 coefficients, L = 32, calls in a row: 139 to
+// 145 us, 3.7 TB/s (762 us for the kernel with 32-bit multiply-add chains);
+// one call by itself 153.  On the way: one-lane issue loop 166 us, TMEM loads of 32
+// columns two deep (spills) 339 us, producers' own proxy fences 181 us.
 #pragma once
 #include <cuda_fp16.h>
 
@@ -371,8 +372,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
       for (uint32_t c = 0; c < NC; ++c) {
         wait(bars, &bars->full[slot], round & 1u, status);
-        // the producers' generic writes before the tensor cores' reads: one
-        // fence here, since a producer's would also wait for its words in flight
+        // The producers' generic writes before the tensor cores' reads.  Their
+        // arrivals release the writes and this wait acquires them; a proxy
+        // fence orders the two proxies wherever it stands between the write
+        // and the read in causality order (PTX memory consistency model), so
+        // one here serves all producers, whose own would each also wait for
+        // their words in flight.
         fence_proxy_async();
         fence_after();
         const uint64_t a0 = desc_a + slot * (kChunkBytes >> 4), b0 = desc_b + c * (image_chunk(N) >> 4);

@@ -222,7 +222,7 @@ int ensure32(int device, uint32_t log_n, uint32_t cm0, uint32_t L, const DevMod3
 template <int LOGN>
 struct Cfg32 {
   static constexpr int T = LOGN > 11 ? LOGN : 11;
-  static constexpr int LOGE = LOGN < 4 ? LOGN : (T == 15 ? 5 : 4);
+  static constexpr int LOGE = LOGN < 4 ? LOGN : 4;
   using C = TileCfg<T, LOGN, 0, LOGE>;
   static constexpr size_t kSmem = Smem<uint32_t>::words(1u << T) * sizeof(uint32_t);
 };
@@ -881,7 +881,7 @@ int host_ntt32(int kind, uint32_t* op, uint32_t log_n, uint32_t cm) {
   const size_t n = (size_t)1 << log_n;
   cudaStream_t s = ctx->stream();
   if (log_n <= kSmallCall32LogN) {
-    // small call: one single-CTA launch in place on the mapped host buffer
+    // small call: one launch in place on the mapped host buffer
     std::lock_guard<std::mutex> g(ctx->small.lock);
     st = ctx->small.ensure();
     if (st != kOk) return st;

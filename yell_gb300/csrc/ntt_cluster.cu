@@ -1,7 +1,8 @@
 // Cluster variants, degrees 2^10 .. 2^14 (k1 = column stages), for calls with
 // few limbs.  GB300, us (before -> here), polymul / forward NTT: 1 limb of
-// 2^10 14.5 -> 5.8 / 8.2 -> 3.8; 8 limbs of 2^12 20.5 -> 6.8 / 10.9 -> 4.4; 10
-// of 2^13 36.9 -> 8.4 / 16.5 -> 5.1; 11 of 2^14 38.7 -> 13.7 / 10.8 -> 6.7.  The
+// 2^10 14.5 -> 5.5 (its NTTs run one limb per CTA); 8 limbs of 2^12 20.5 -> 6.7 /
+// 10.9 -> 4.2; 10 of 2^13 36.9 -> 8.2 / 16.5 -> 4.7; 15 of 2^13 36.9 -> 9.9; 11 of
+// 2^14 38.7 -> 13.5 / 10.8 -> 6.4.  The
 // ranges end where another variant is as fast: 2^10 polymul at 96 limbs 7.1
 // against 6.4 with one limb per CTA; 2^11 at 2048 103.6 against 100.3; 2^12 on
 // 8 CTAs and on 4: polymul at 16 limbs 7.7 and 7.6, NTT at 64 6.0 and 5.7, at

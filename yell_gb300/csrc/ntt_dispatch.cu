@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(256) k_elementwise(LimbSet dst, ConstLimbSet a
   constexpr int kPairs = ew_product(OP) || !kBinary ? 1 : 2;
   constexpr bool kAcc = OP == (int)EwOp::kMuladd;
   grid_dep_launch();
-  grid_dep_wait();  // as in the two-pass kernels
+  grid_dep_wait();  // the caller's words, and its limb and modulus lists, come after
   const size_t pairs = ((size_t)dst.count << log_n) >> 1;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const uint32_t nmask = (1u << log_n) - 1u;

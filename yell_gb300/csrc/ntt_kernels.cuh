@@ -1,10 +1,10 @@
 // NTT and fused polymul kernels for sm_103a (templates; see ntt_variants.h).
 //
 // Paths (per degree N = 2^log_n):
-//   * whole-limb: N <= 2^13.  One CTA holds whole limbs in shared memory
-//     (several limbs per CTA below 2^12), reads each word from HBM once and
-//     writes it once.
-//   * two-pass: N >= 2^14.  N = C x B with C = 2^k1.  The column pass applies
+//   * whole-limb: N <= 2^12, and 2^13 without scratch.  One CTA holds whole
+//     limbs in shared memory (several limbs per CTA below 2^12, one for calls
+//     of few limbs), reads each word from HBM once and writes it once.
+//   * two-pass: N >= 2^13.  N = C x B with C = 2^k1.  The column pass applies
 //     forward stages 0..k1-1, which pair words B*2^t apart (columns of stride
 //     B); the row pass applies stages k1..log_n-1, which stay inside
 //     contiguous blocks of B words.  The inverse runs the same passes in the
@@ -38,7 +38,7 @@ namespace yell_gb300 {
 // this header instantiates the kernels of its own degrees and variants.
 namespace {
 
-constexpr int kTileLog = 12;  // 4096 words per two-pass tile
+constexpr int kTileLog = 12;  // 4096 words: two-pass tiles unless TwoPassTiles or a variant for few limbs says otherwise
 
 // The caller's words, and those of a pass before.  The read-only path (__ldg)
 // is for memory that nobody writes while the kernel runs, and a kernel launched
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(C::THREADS, min_blocks(INV ? 1024 : 768, C::TH
 }
 
 // ===========================================================================
-// Two-pass row pass over 4096 contiguous words (2^(12-K) blocks of 2^K).
+// Two-pass row pass over a tile of 2^T contiguous words (2^(T-K) blocks of 2^K).
 // Forward: stages k1..log_n-1 (+ the final reduction when reduce); inverse:
 // stages 0..K-1.  In place.
 // ===========================================================================
@@ -1025,8 +1025,8 @@ cudaError_t set_smem(KernelT kernel, size_t bytes) {
 constexpr int whole_loge(int log_n) { return log_n >= 4 ? 4 : 3; }
 template <int LOGN, int T, int LOGE = whole_loge(LOGN)>
 using WholeCfg = TileCfg<T, LOGN, 0, LOGE>;
-// Two-pass tiles: 4096 words, 2^LOGE words per thread per round (radix-2^LOGE
-// rounds): LOGE = 4 is 256 threads, LOGE = 3 is 512 threads per tile.
+// Two-pass tiles: 2^T words, 2^LOGE words per thread per round (radix-2^LOGE
+// rounds): a tile of 2^12 is 256 threads at LOGE = 4, 512 at LOGE = 3.
 template <int LOGN, int K1, int LOGE = 4, int T = kTileLog>
 using ColCfg = TileCfg<T, K1, T - K1, LOGE>;
 template <int LOGN, int K1, int LOGE = 4, int T = kTileLog>
@@ -1084,8 +1084,8 @@ cudaError_t set_attrs_whole() {
 // 2^16 at k1 = 7, tiles of 2^12 with 16 words per thread -> the tile below:
 // forward column pass 156 -> 144 us (147 at 2^11 words, which k1 = 6 and 8
 // prefer: 138 and 160 against 141 and 162), forward row pass 225 -> 206,
-// inverse row pass 276 -> 233, inverse column pass 173 -> 163 (polymul 170 ->
-// 160), polymul's forward column pass 291 -> 284 (8 words, compiled for 1024
+// inverse row pass 276 -> 233, inverse column pass 173 -> 156 (polymul 170 ->
+// 154), polymul's forward column pass 291 -> 284 (8 words, compiled for 1024
 // threads per SM; 286 for 896, 296 for 768; at k1 = 6 290 -> 250); 512 limbs
 // of 2^14: 87 -> 78.  2^13 keeps 768 threads (64 limbs: 10.1 us against 11.1).
 // Only the fused row step (16 words of two operands per thread) wants its 2^12

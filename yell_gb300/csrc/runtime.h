@@ -49,8 +49,8 @@ void load_tuning(int device);
 int check_degree(uint32_t log_n);
 int check_moduli(uint32_t cm0, uint32_t L);
 // count polys (or pairs) of L limbs each: rejects a zero count and a limb
-// total of one call that would not fit its launch grid (in particular any
-// count * L >= 2^32).  On success *limbs = count * L (when limbs != nullptr).
+// total beyond 2^31 limbs or 4096-word tiles (in particular any count * L >=
+// 2^32).  On success *limbs = count * L (when limbs != nullptr).
 int check_limbs(uint64_t count, uint32_t L, uint32_t log_n, uint32_t* limbs);
 
 // Looks up, once per device, the device address of the fixed scratch array
