@@ -438,9 +438,12 @@ __global__ void __launch_bounds__(C::THREADS, min_blocks(INV ? 1024 : 768, C::TH
   const uint64_t* in = src.limb(limb, log_n) + col0;
   uint64_t* out = dst.limb(limb, log_n) + col0;
   uint64_t x[1 << C::LOGE];
-  // the inverse requests its words first: 512 limbs of 2^16 at k1 = 7 153.7 us
-  // against 161.5 with the constants first
-  if constexpr (INV) {
+  // the inverse at 16 words per thread requests its words first: 512 limbs of
+  // 2^16 at k1 = 7 153.7 us against 161.5 with the constants first.  The tiles
+  // of few limbs are latency bound, and their twiddles wait for the constants
+  // (whole inverse of 4 limbs of 2^16 7.74 us words first, 7.56 constants first)
+  constexpr bool kWordsFirst = INV && C::LOGE == 4;
+  if constexpr (kWordsFirst) {
     using RB = Round<C, NR - 1>;
     gload_cols<RB, LOGB>(x, in, RB::base(tid));
   }
@@ -465,6 +468,7 @@ __global__ void __launch_bounds__(C::THREADS, min_blocks(INV ? 1024 : 768, C::TH
   } else {
     using RB = Round<C, NR - 1>;  // bottom round, executed first
     const uint32_t bb = RB::base(tid);
+    if constexpr (!kWordsFirst) gload_cols<RB, LOGB>(x, in, bb);
     if constexpr (NR == 1) {
       gs_round<RB, true>(x, log_n, LOGB + RB::BETA, RB::gr(bb, 0), m);
       gstore_cols<RB, LOGB>(x, out, bb);
