@@ -55,6 +55,22 @@ __device__ __forceinline__ uint64_t ld_word(const uint64_t* p) {
   return v;
 }
 
+__device__ __forceinline__ uint4 ld_quad(const uint32_t* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint2 ld_pair(const uint32_t* p) {
+  uint2 v;
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_word(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
 // Loads of words another CTA of the same launch wrote (the persistent batch
 // kernel's intermediates): through L2.
 __device__ __forceinline__ ulonglong2 ld_pair_cg(const uint64_t* p) {
@@ -76,12 +92,12 @@ __device__ __forceinline__ ulonglong2 ld_pair_t(const uint64_t* p) {
 template <bool COH>
 __device__ __forceinline__ uint2 ld_pair_t(const uint32_t* p) {
   static_assert(!COH, "no 32-bit kernel reads words of its own launch");
-  return *reinterpret_cast<const uint2*>(p);
+  return ld_pair(p);
 }
 template <bool COH>
 __device__ __forceinline__ uint32_t ld_word_t(const uint32_t* p) {
   static_assert(!COH, "no 32-bit kernel reads words of its own launch");
-  return *p;
+  return ld_word(p);
 }
 template <bool COH>
 __device__ __forceinline__ uint64_t ld_word_t(const uint64_t* p) {
@@ -115,7 +131,7 @@ __device__ __forceinline__ void gload_rows(W* x, const W* g, uint32_t base_u) {
   } else if constexpr (RG::CONTIG && sizeof(W) == 4 && R >= 2) {
 #pragma unroll
     for (int j = 0; j < (1 << R); j += 4) {
-      const uint4 v = *reinterpret_cast<const uint4*>(gb + j);
+      const uint4 v = ld_quad(gb + j);
       x[j] = v.x;
       x[j + 1] = v.y;
       x[j + 2] = v.z;
