@@ -12,7 +12,7 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 def test_allocation_between_wait_and_launch():
     text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "crt_mma.cuh")).read())
     body = text[text.index("k_crt_mma("):]
-    steps = ["grid_dep_wait()", "tcgen05.alloc", "__syncthreads()", "grid_dep_launch()", "tcgen05.dealloc"]
+    steps = ["grid_dep_wait()", "tcgen05.alloc", "tmem_address(bars)", "grid_dep_launch()", "tcgen05.dealloc"]
     at = [body.index(s) for s in steps]
     assert at == sorted(at), dict(zip(steps, at))
     assert all(body.count(s) == 1 for s in ("grid_dep_wait()", "tcgen05.alloc", "grid_dep_launch()"))

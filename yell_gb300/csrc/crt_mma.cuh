@@ -185,6 +185,15 @@ __device__ __forceinline__ void wait(Bars* b, uint64_t* mbar, uint32_t parity, u
   if (!mbar_test(mbar, parity)) wait_slow<LIMIT>(b, mbar, parity, status);
 }
 
+// The TMEM address that the issuing warp's allocation left, for that warp and
+// the epilogue's.
+__device__ __forceinline__ uint32_t tmem_address(Bars* b) {
+  fence_before();
+  asm volatile("bar.sync 2, %0;" ::"n"(32 * (kEpilogueWarps + 1)) : "memory");
+  fence_after();
+  return *(volatile uint32_t*)&b->tmem;
+}
+
 // Check of the bounded wait: one CTA waits twice on a barrier at which nobody
 // arrives.  The first wait runs out and records YELL_ERR_TIMEOUT, the second
 // returns at once.
@@ -243,24 +252,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     mbar_init(&bars->done, 1);
     bars->gave_up = 0;
   }
-  // The caller's words are read and written below.  TMEM is taken only now:
-  // a CTA that holds columns while it waits could keep them from a CTA of the
-  // kernel that it waits for.  For the same reason the next kernel may start
-  // only once this CTA has its columns.
-  grid_dep_wait();
-  if (warp == kEpilogueWarps + kProducerWarps) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     (uint32_t)__cvta_generic_to_shared(&bars->tmem)),
-                 "r"(tmem_cols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
   fence_proxy_async();
-  fence_before();
   __syncthreads();
-  fence_after();
-  grid_dep_launch();
-  const uint32_t tmem = *(volatile uint32_t*)&bars->tmem;
+  grid_dep_wait();  // the caller's words are read and written below
 
   if (warp >= kEpilogueWarps && warp < kEpilogueWarps + kProducerWarps) {
     // ---- producers: thread (row, part) takes moduli 8 c + kMine part .. of each chunk c
@@ -357,6 +351,17 @@ __global__ void __launch_bounds__(kThreads, 1)
     // the same values, so the operand descriptors stay in uniform registers,
     // and one lane issues: with the whole loop inside a one-lane branch an MMA
     // took 220 cycles to issue (128 to run) beside the producers' warps.
+    //
+    // TMEM is taken only now, while the producers start: a CTA that holds columns
+    // while it waits could keep them from a CTA of the kernel that it waits for.
+    // For the same reason the next kernel may start only once this CTA has them.
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(&bars->tmem)),
+                 "r"(tmem_cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    const uint32_t tmem = tmem_address(bars);
+    grid_dep_launch();
     const uint32_t idesc = (1u << 4) | ((N >> 3) << 17) | ((kRows >> 4) << 24);  // f16 x f16 -> f32, both K-major
     const uint64_t desc_a = operand_desc(s_addr + lay.ring, 1024, kSwizzle128);
     const uint64_t desc_b = operand_desc(s_addr, 1024, kSwizzle128);
@@ -414,6 +419,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else {
     // ---- epilogue: warps 4 b .. 4 b + 3 take the tiles of accumulator b; thread
     // = coefficient row 32 * quarter + lane = TMEM lane
+    const uint32_t tmem = tmem_address(bars);
     const uint32_t quarter = warp & 3u, b = warp >> 2, row = quarter * 32 + lane;
     uint64_t* stage = reinterpret_cast<uint64_t*>(s + lay.stage) + warp * 32 * kStageStride;
     uint32_t kt = 0, t = b;
@@ -508,6 +514,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   if (warp == kEpilogueWarps + kProducerWarps) {
     fence_after();
+    const uint32_t tmem = *(volatile uint32_t*)&bars->tmem;
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols) : "memory");
   }
 }
