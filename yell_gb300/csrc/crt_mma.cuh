@@ -185,11 +185,12 @@ __device__ __forceinline__ void wait(Bars* b, uint64_t* mbar, uint32_t parity, u
   if (!mbar_test(mbar, parity)) wait_slow<LIMIT>(b, mbar, parity, status);
 }
 
-// The TMEM address that the issuing warp's allocation left, for that warp and
-// the epilogue's.
+// The TMEM address that the issuing warp's allocation left.  All threads of the
+// CTA meet here, so that no bounded wait runs while another kernel on this SM
+// still has the columns.
 __device__ __forceinline__ uint32_t tmem_address(Bars* b) {
   fence_before();
-  asm volatile("bar.sync 2, %0;" ::"n"(32 * (kEpilogueWarps + 1)) : "memory");
+  asm volatile("bar.sync 2, %0;" ::"n"(kThreads) : "memory");
   fence_after();
   return *(volatile uint32_t*)&b->tmem;
 }
@@ -281,6 +282,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     locate(blockIdx.x);
 #pragma unroll
     for (uint32_t c = 0; c < NC; ++c) fetch(c);
+    (void)tmem_address(bars);
     uint32_t slot = 0, round = 0, t = 0, ts = 0, tr = 0;
     // this thread's 16-byte units of a chunk row
     uint8_t* unit[kMine];
