@@ -460,7 +460,7 @@ int crt_lift(uint64_t* d_out, const uint64_t* d_in, uint32_t count, uint32_t L, 
   // From 4 moduli up the tensor-core kernel is the faster one at every number
   // of coefficients (GB300, us, digit kernel -> tensor cores: 2^20
   // coefficients, L = 3: 33 -> 41, 4: 53 -> 38, 8: 117 -> 47, 16: 286 -> 78,
-  // 32: 762 -> 139; 2^13, L = 3: 3.7 -> 4.1, 32: 35 -> 6); its digits are exact
+  // 32: 762 -> 137; 2^13, L = 3: 3.7 -> 4.1, 32: 35 -> 5.7); its digits are exact
   // up to kMaxL moduli.
   if (t->image) {
     const cudaError_t me = launch_crt_mma(d_out, d_in, (uint64_t)count << log_n, L, log_n, t, st, device, own_status);

@@ -36,10 +36,10 @@
 //
 // What bounds it: no one unit.  Per tile at L = 32 the tensor cores need 2190
 // cycles, HBM (63 words per coefficient) 3000, and a tile takes about 5000;
-// the counters have issue slots at 48%, the tensor pipe at 37%, DRAM at 22%,
+// the counters have issue slots at 49%, the tensor pipe at 38%, DRAM at 23%,
 // and warps waiting on long scoreboards, fixed latencies and the barriers
-// between them.  GB300, 16 x 2^16 coefficients, L = 32, calls in a row: 139 to
-// 145 us, 3.7 TB/s (762 us for the kernel with 32-bit multiply-add chains);
+// between them.  GB300, 16 x 2^16 coefficients, L = 32, calls in a row: 136 to
+// 142 us, 3.8 TB/s (762 us for the kernel with 32-bit multiply-add chains);
 // one call by itself 153.  On the way: one-lane issue loop 166 us, TMEM loads of 32
 // columns two deep (spills) 339 us, producers' own proxy fences 181 us.
 #pragma once
