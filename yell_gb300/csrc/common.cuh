@@ -352,7 +352,8 @@ template <> struct PairOf<uint32_t> {
 // and the running kernel's were packed onto what was left (GB300, polymul of 2
 // limbs of 2^15: 15.9 us with the launch before the wait, 10.7 after; 1 of
 // 2^16 17.2 and 10.6; NTT of 3 limbs of 2^16 9.5 and 7.5).  In the samplers and
-// the element-wise ops the order made no difference; they call it first.
+// the element-wise ops the order made no difference; they call it first.  The
+// tensor-core CRT lift calls it once it has its tensor memory (crt_mma.cuh).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -40,7 +40,7 @@
 // and warps waiting on long scoreboards, fixed latencies and the barriers
 // between them.  GB300, 16 x 2^16 coefficients, L = 32, calls in a row: 136 to
 // 142 us, 3.8 TB/s (762 us for the kernel with 32-bit multiply-add chains);
-// one call by itself 153.  On the way: one-lane issue loop 166 us, TMEM loads of 32
+// one call by itself 151.  On the way: one-lane issue loop 166 us, TMEM loads of 32
 // columns two deep (spills) 339 us, producers' own proxy fences 181 us.
 #pragma once
 #include <cuda_fp16.h>
